@@ -28,7 +28,7 @@ using swrx::f3;
 using swrx::mk;
 
 constexpr uint32_t kDead = 0xFFFFFFFFu;
-constexpr int kTB = 128;
+constexpr int kTB = swrx::kTraceThreads;
 constexpr double kFix = 4294967296.0;  // 2^32
 // batches of at least this many samples run as kBatchSubWaves concurrent sub-wavefronts
 constexpr uint64_t kBatchTwoWaveSamples = 1ull << 20;
@@ -102,11 +102,12 @@ __device__ __forceinline__ uint32_t find_job(const BJob* jobs, uint32_t n, uint6
 // the pixel-centre ray; a back-facing first hit restarts the lane's traversal past it (using up a
 // depth slot), so lanes do not wait for the warp's slowest pixel.
 __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ctrl) {
-  __shared__ uint2 stack[swrx::kStackShared * kTB];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTB];
   const unsigned ln = lane();
   const unsigned lt = (1u << ln) - 1u;
   const unsigned refill = A.refill ? A.refill : 8u;
   swrx::Traversal tr;
+  tr.setup(stack);
   const DevScene* sc = nullptr;
   bool active = false, exhausted = false;
   uint64_t p = 0;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ct
           depth = J.depth;
           const uint32_t pix = (uint32_t)(p - J.pixel_base);
           d = swrx::primary_dir(J.vi, J.pi, pix % J.W, pix / J.W, J.W, J.H);
-          tr.init(mk(J.org[0], J.org[1], J.org[2]), d, stack + threadIdx.x, kTB);
+          tr.init(mk(J.org[0], J.org[1], J.org[2]), d, stack);
           ++traced;
           active = true;
         }
@@ -141,24 +142,28 @@ __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ct
       if (exhausted) break;
       continue;
     }
-    if (active && tr.step<false>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, nullptr)) {
+    if (active && tr.step<false>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
+      if (!tr.settled(sc->tris, sc->tri_boxes, sc->obj_boxes, stack)) {
+        tr.start_strict(stack);
+        continue;
+      }
       // depth slot i traced: a miss ends the prefix, a back face uses up the slot
       float4 r0 = make_float4(0, 0, 0, 0), r1 = make_float4(0, 0, 0, __uint_as_float(kDead));
       bool done = true;
-      if (tr.hit.slot != 0xFFFFFFFFu) {
+      if (tr.hit_slot(stack) != 0xFFFFFFFFu) {
         const f3 o = tr.o;
-        const f3 hp = swrx::hit_point(o, d, tr.hit.t);
-        const f3 n = swrx::shading_normal(sc->tris, sc->shade, tr.hit.slot, hp);
+        const f3 hp = swrx::hit_point(o, d, tr.hit_t(stack));
+        const f3 n = swrx::shading_normal(sc->tris, sc->shade, tr.hit_slot(stack), hp);
         if (swrx::vdot(n, d) > 0.0f) {
           if (i + 1 < depth) {
-            tr.init(swrx::vadd(hp, swrx::vscale(0.01f, d)), d, stack + threadIdx.x, kTB);
+            tr.init(swrx::vadd(hp, swrx::vscale(0.01f, d)), d, stack);
             ++i;
             ++traced;
             done = false;
           }
         } else {
-          r0 = make_float4(o.x, o.y, o.z, tr.hit.t);
-          r1 = make_float4(d.x, d.y, d.z, __uint_as_float(tr.hit.slot | (i << 27)));
+          r0 = make_float4(o.x, o.y, o.z, tr.hit_t(stack));
+          r1 = make_float4(d.x, d.y, d.z, __uint_as_float(tr.hit_slot(stack) | (i << 27)));
         }
       }
       if (done) {
@@ -323,8 +328,8 @@ __global__ void __launch_bounds__(256) k_bshade(BArgs A, BCtrl* __restrict__ ctr
 }
 
 // bounce traversal over the shared queue, refilling idle lanes (as the single-scene kernel)
-__global__ void __launch_bounds__(kTB) k_btrace(BArgs A, BCtrl* __restrict__ ctrl, BQueue q, int parity) {
-  __shared__ uint2 stack[swrx::kStackShared * kTB];
+__global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ ctrl, BQueue q, int parity) {
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTB];
   const int qp = parity ^ 1;
   const unsigned n = ctrl->count[qp];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -340,25 +345,39 @@ __global__ void __launch_bounds__(kTB) k_btrace(BArgs A, BCtrl* __restrict__ ctr
   const unsigned ln = lane();
   const unsigned lt = (1u << ln) - 1u;
   swrx::Traversal tr;
+  tr.setup(stack);
   const DevScene* sc = nullptr;
   bool active = false, exhausted = false;
-  unsigned ray = 0;
+  bool unwritten = false;  // the lane is idle and its finished ray (row kRowUser) is not written yet
   for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    if (!exhausted && (unsigned)__popc(idle) >= A.refill) {
-      unsigned base = 0;
-      if (ln == 0) base = atomicAdd(&ctrl->cursor[qp], (unsigned)__popc(idle));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= n) exhausted = true;
-      if (!active) {
-        const unsigned j = base + __popc(idle & lt);
-        if (j < n) {
-          const float4 o = q.o[j], d = q.d[j];
-          const uint32_t job = __float_as_uint(q.c[j].w) >> 16;
-          sc = &A.scenes[A.jobs[job].scene];
-          tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack + threadIdx.x, kTB);
-          ray = j;
+    unsigned idle = __ballot_sync(0xffffffffu, !active);
+    if (exhausted ? idle == 0xffffffffu : (unsigned)__popc(idle) >= A.refill) {
+      // settle and write the finished rays together
+      if (unwritten) {
+        unwritten = false;
+        if (tr.settled(sc->tris, sc->tri_boxes, sc->obj_boxes, stack)) {
+          q.hit[tr.st.get(stack, swrx::kRowUser).x] = tr.st.get(stack, swrx::kRowHit);
+        } else {
+          tr.start_strict(stack);
           active = true;
+        }
+      }
+      idle = __ballot_sync(0xffffffffu, !active);
+      if (!exhausted) {
+        unsigned base = 0;
+        if (ln == 0) base = atomicAdd(&ctrl->cursor[qp], (unsigned)__popc(idle));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= n) exhausted = true;
+        if (!active) {
+          const unsigned j = base + __popc(idle & lt);
+          if (j < n) {
+            const float4 o = q.o[j], d = q.d[j];
+            const uint32_t job = __float_as_uint(q.c[j].w) >> 16;
+            sc = &A.scenes[A.jobs[job].scene];
+            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack);
+            tr.st.set(stack, swrx::kRowUser, make_uint2(j, 0u));
+            active = true;
+          }
         }
       }
     }
@@ -366,9 +385,9 @@ __global__ void __launch_bounds__(kTB) k_btrace(BArgs A, BCtrl* __restrict__ ctr
       if (exhausted) break;
       continue;
     }
-    if (active && tr.step<false, false>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, nullptr)) {
-      q.hit[ray] = make_uint2(tr.hit.slot, __float_as_uint(tr.hit.t));
+    if (active && tr.step<false, false>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
       active = false;
+      unwritten = true;
     }
   }
 }
@@ -379,11 +398,12 @@ __global__ void __launch_bounds__(kTB) k_btrace(BArgs A, BCtrl* __restrict__ ctr
 // per-pixel camera record and replay the path with the job's scene, seed and Russian roulette,
 // then sweep it into the job's gradient buffers. ctrl->injected is the sample cursor.
 __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ ctrl) {
-  __shared__ uint2 stack[swrx::kStackShared * kTB];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTB];
   const unsigned ln = lane();
   const unsigned lt = (1u << ln) - 1u;
   const unsigned long long total = ctrl->total;
   swrx::Traversal tr;
+  tr.setup(stack);
   swrx::PathState st;
   swrx::AdjointTape tape;
   tape.reset();
@@ -419,6 +439,7 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
             st.v = 0;
             pend_slot = bits & 0x07FFFFFFu;
             pend_t = r0.w;
+            tr.no_hit(stack);  // the camera record's hit is settled
             tape.reset();
             tracing = false;
             active = true;
@@ -430,13 +451,13 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, nullptr)) {
+    if (active && tracing && tr.step<false, false>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
       tracing = false;
-      if (tr.hit.slot == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
+      if (tr.hit_slot(stack) == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
         active = false;
       } else {
-        pend_slot = tr.hit.slot;
-        pend_t = tr.hit.t;
+        pend_slot = tr.hit_slot(stack);
+        pend_t = tr.hit_t(stack);
       }
     }
     // lanes with a pending hit wait until A.batch of them (or every active lane) shade together
@@ -444,6 +465,11 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);
     if (waiting == 0u || ((unsigned)__popc(waiting) < A.batch && inflight != 0u)) continue;
     if (!active || tracing) continue;
+    if (!tr.settled(sc->tris, sc->tri_boxes, sc->obj_boxes, stack)) {
+      tr.start_strict(stack);
+      tracing = true;
+      continue;
+    }
     swrx::ShadeParams P;
     P.seed = J->seed;
     P.pixel = pixel;
@@ -458,7 +484,7 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
         swrx::shade_physical_adj(sc->tris, sc->shade, sc->mats, sc->albedo, pend_slot, pend_t, P, st, av);
     if (outcome == swrx::kContinue) {
       tape.push(pend_slot, c_before, av);
-      tr.init(st.o, st.d, stack + threadIdx.x, kTB);
+      tr.init(st.o, st.d, stack);
       tracing = true;
       continue;
     }

@@ -20,6 +20,7 @@
 #include <cstring>
 #include <vector>
 
+#include "../plane_grid.h"
 #include "build_device.h"
 #include "swr_internal.cuh"
 
@@ -383,22 +384,8 @@ __global__ void k_emit(EmitArgs A, const Task* __restrict__ tasks, uint32_t ntas
       child_in_slot[bsi] = bci;
     }
   }
-  // quantisation grid: per axis the smallest power of two e with 255 e >= extent
-  uint32_t ebyte[3];
-  double e[3];
-  for (int k = 0; k < 3; ++k) {
-    const double ext = (double)uhi[k] - (double)ulo[k];
-    int ex = -126;
-    if (ext > 0.0) {
-      int x;
-      frexp(ext / 255.0, &x);
-      ex = x;
-      if (ldexp(1.0, ex - 1) >= ext / 255.0) ex = ex - 1;
-    }
-    ex = max(-126, min(127, ex));
-    ebyte[k] = (uint32_t)(ex + 127);
-    e[k] = ldexp(1.0, ex);
-  }
+  swrx::PlaneGrid grid[3];
+  for (int k = 0; k < 3; ++k) grid[k] = swrx::plane_grid(ulo[k], uhi[k]);
   // triangles of the leaf children and the count of inner children
   uint32_t leaf_tris[8];
   uint32_t n_inner = 0, n_tris = 0;
@@ -430,10 +417,8 @@ __global__ void k_emit(EmitArgs A, const Task* __restrict__ tasks, uint32_t ntas
     const int ci = child_in_slot[s];
     if (ci < 0) continue;
     for (int k = 0; k < 3; ++k) {
-      const double lo = floor(((double)cb[ci].lo[k] - (double)ulo[k]) / e[k]);
-      const double hi = ceil(((double)cb[ci].hi[k] - (double)ulo[k]) / e[k]);
-      qlo[k][s] = (uint8_t)fmax(0.0, fmin(255.0, lo));
-      qhi[k][s] = (uint8_t)fmax(0.0, fmin(255.0, hi));
+      qlo[k][s] = (uint8_t)swrx::plane_below(grid[k], cb[ci].lo[k]);
+      qhi[k][s] = (uint8_t)swrx::plane_above(grid[k], cb[ci].hi[k]);
     }
     const uint32_t v = ch[ci];
     if (leaf_tris[s]) {
@@ -465,10 +450,8 @@ __global__ void k_emit(EmitArgs A, const Task* __restrict__ tasks, uint32_t ntas
     }
   }
   uint32_t* w = A.words + (size_t)tk.wide * 20;
-  w[0] = __float_as_uint(ulo[0]);
-  w[1] = __float_as_uint(ulo[1]);
-  w[2] = __float_as_uint(ulo[2]);
-  w[3] = ebyte[0] | (ebyte[1] << 8) | (ebyte[2] << 16) | (imask << 24);
+  for (int k = 0; k < 3; ++k) w[k] = __float_as_uint(grid[k].origin);
+  w[3] = grid[0].ebyte | (grid[1].ebyte << 8) | (grid[2].ebyte << 16) | (imask << 24);
   w[4] = child_base;
   w[5] = tri_base;
   w[6] = meta[0] | (meta[1] << 8) | (meta[2] << 16) | ((uint32_t)meta[3] << 24);

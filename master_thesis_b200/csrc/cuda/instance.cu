@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "../host/capi_common.h"
+#include "../plane_grid.h"
 #include "swr_internal.cuh"
 
 namespace swr {
@@ -338,23 +339,9 @@ __global__ void k_refit(InstView I, uint32_t* __restrict__ words, uint32_t begin
       }
     }
   }
-  // quantisation grid of the builder: per axis the smallest power of two e with 255 e >= extent
-  uint32_t ebyte[3];
-  double e[3];
+  swrx::PlaneGrid grid[3];  // as the builder's
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const double ex_d = (double)uhi[q] - (double)ulo[q];
-    int ex = -126;
-    if (ex_d > 0.0) {
-      int x;
-      frexp(ex_d / 255.0, &x);
-      ex = x;
-      if (ldexp(1.0, ex - 1) >= ex_d / 255.0) ex = ex - 1;
-    }
-    ex = max(-126, min(127, ex));
-    ebyte[q] = (uint32_t)(ex + 127);
-    e[q] = ldexp(1.0, ex);
-  }
+  for (int q = 0; q < 3; ++q) grid[q] = swrx::plane_grid(ulo[q], uhi[q]);
   uint32_t qlo[3][2] = {{0, 0}, {0, 0}, {0, 0}}, qhi[3][2] = {{0, 0}, {0, 0}, {0, 0}};
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
@@ -362,19 +349,16 @@ __global__ void k_refit(InstView I, uint32_t* __restrict__ words, uint32_t begin
     for (int q = 0; q < 3; ++q) {
       uint32_t l = 255u, h = 0u;
       if (used[s]) {
-        const double lo = floor(((double)clo[s][q] - (double)ulo[q]) / e[q]);
-        const double hi = ceil(((double)chi[s][q] - (double)ulo[q]) / e[q]);
-        l = (uint32_t)fmax(0.0, fmin(255.0, lo));
-        h = (uint32_t)fmax(0.0, fmin(255.0, hi));
+        l = swrx::plane_below(grid[q], clo[s][q]);
+        h = swrx::plane_above(grid[q], chi[s][q]);
       }
       qlo[q][s >> 2] |= l << (8 * (s & 3));
       qhi[q][s >> 2] |= h << (8 * (s & 3));
     }
   }
-  w[0] = __float_as_uint(ulo[0]);
-  w[1] = __float_as_uint(ulo[1]);
-  w[2] = __float_as_uint(ulo[2]);
-  w[3] = ebyte[0] | (ebyte[1] << 8) | (ebyte[2] << 16) | (imask << 24);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) w[q] = __float_as_uint(grid[q].origin);
+  w[3] = grid[0].ebyte | (grid[1].ebyte << 8) | (grid[2].ebyte << 16) | (imask << 24);
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     w[8 + 2 * q] = qlo[q][0];

@@ -30,7 +30,7 @@ using swrx::f3;
 using swrx::mk;
 
 constexpr uint32_t kDeadSlot = 0xFFFFFFFFu;
-constexpr int kTraceBlock = 128;
+constexpr int kTraceBlock = swrx::kTraceThreads;
 constexpr uint64_t kChunkSamples = 1ull << 27;
 // chunks of at least this many samples, on scenes of at least kTwoWaveTriangles triangles, run as
 // kSubWaves concurrent sub-wavefronts (SWR_RENDER_ONE_WAVEFRONT). Measured on B200: 28.02 vs 28.49
@@ -94,12 +94,13 @@ __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 // restarts it 0.01 further along the ray; when at least F.refill lanes of the warp are idle they
 // take that many new pixels from the chunk's pixel cursor with one atomic.
 __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ctrl* __restrict__ ctrl) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const unsigned lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   const unsigned refill = F.refill ? F.refill : 8u;
   const f3 org = mk(F.org[0], F.org[1], F.org[2]);
   swrx::Traversal tr;
+  tr.setup(stack);
   bool active = false, exhausted = false;
   uint32_t k = 0, i = 0;
   f3 d = mk(0.0f, 0.0f, 0.0f);
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
           i = 0;
           const uint32_t pix = F.pixel0 + k;
           d = swrx::primary_dir(F.vi, F.pi, pix % F.W, pix / F.W, F.W, F.H);
-          tr.init(org, d, stack + threadIdx.x, kTraceBlock);
+          tr.init(org, d, stack);
           ++traced;
           active = true;
         }
@@ -128,24 +129,28 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
       if (exhausted) break;
       continue;
     }
-    if (active && tr.template step<false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, nullptr)) {
+    if (active && tr.template step<false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
+      if (!tr.settled(sc.tris, sc.tri_boxes, sc.obj_boxes, stack)) {
+        tr.start_strict(stack);
+        continue;
+      }
       // depth slot i traced: a miss ends the prefix, a back face uses up the slot
       float4 rec0 = make_float4(0, 0, 0, 0), rec1 = make_float4(0, 0, 0, __uint_as_float(kDeadSlot));
       bool done = true;
-      if (tr.hit.slot != 0xFFFFFFFFu) {
+      if (tr.hit_slot(stack) != 0xFFFFFFFFu) {
         const f3 o = tr.o;
-        const f3 p = swrx::hit_point(o, d, tr.hit.t);
-        const f3 n = swrx::shading_normal(sc.tris, sc.shade, tr.hit.slot, p);
+        const f3 p = swrx::hit_point(o, d, tr.hit_t(stack));
+        const f3 n = swrx::shading_normal(sc.tris, sc.shade, tr.hit_slot(stack), p);
         if (swrx::vdot(n, d) > 0.0f) {
           if (i + 1 < F.depth) {
-            tr.init(swrx::vadd(p, swrx::vscale(0.01f, d)), d, stack + threadIdx.x, kTraceBlock);
+            tr.init(swrx::vadd(p, swrx::vscale(0.01f, d)), d, stack);
             ++i;
             ++traced;
             done = false;
           }
         } else {
-          rec0 = make_float4(o.x, o.y, o.z, tr.hit.t);
-          rec1 = make_float4(d.x, d.y, d.z, __uint_as_float(tr.hit.slot | (i << 27)));
+          rec0 = make_float4(o.x, o.y, o.z, tr.hit_t(stack));
+          rec1 = make_float4(d.x, d.y, d.z, __uint_as_float(tr.hit_slot(stack) | (i << 27)));
         }
       }
       if (done) {
@@ -355,7 +360,7 @@ static unsigned shade_grid_for(const swr_scene* s, uint32_t cap, int block) {
 template <bool kStats>
 __global__ void __launch_bounds__(kTraceBlock)
     k_trace(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   // parity p: trace queue p^1, prepare the injection window of the next shade (parity p^1)
   const int qp = parity ^ 1;
   const unsigned n = ctrl->count[qp];
@@ -371,6 +376,7 @@ __global__ void __launch_bounds__(kTraceBlock)
     ctrl->bounce_rays += n;
     if (ctrl->first_n == 0u) ctrl->first_n = n;
   }
+  swrx::Traversal::prepare(stack);
   swrx::TraceStats st{0, 0};
   for (;;) {
     unsigned base = 0;
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kTraceBlock)
       const float4 o = q.o[i], d = q.d[i];
       swrx::Hit h;
       swrx::trace_closest<kStats>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z),
-                                  mk(d.x, d.y, d.z), stack + threadIdx.x, kTraceBlock, h, &st);
+                                  mk(d.x, d.y, d.z), stack, kTraceBlock, h, &st);
       q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
     }
   }
@@ -407,7 +413,7 @@ __global__ void __launch_bounds__(kTraceBlock)
 template <bool kStats, int kMinBlocks, bool kPostpone>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_trace_dyn(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const int qp = parity ^ 1;
   const unsigned n = ctrl->count[qp];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -426,22 +432,36 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
   const unsigned lt = (1u << lane) - 1u;
   swrx::TraceStats st{0, 0};
   swrx::Traversal tr;
+  tr.setup(stack);
   bool active = false, exhausted = false;
-  unsigned ray = 0;
+  bool unwritten = false;  // the lane is idle and its finished ray (row kRowUser) is not written yet
   for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    if (!exhausted && (unsigned)__popc(idle) >= F.refill) {
-      unsigned base = 0;
-      if (lane == 0) base = atomicAdd(&ctrl->cursor[qp], (unsigned)__popc(idle));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= n) exhausted = true;
-      if (!active) {
-        const unsigned j = base + __popc(idle & lt);
-        if (j < n) {
-          const float4 o = __ldcs(q.o + j), d = __ldcs(q.d + j);
-          tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack + threadIdx.x, kTraceBlock);
-          ray = j;
+    unsigned idle = __ballot_sync(0xffffffffu, !active);
+    if (exhausted ? idle == 0xffffffffu : (unsigned)__popc(idle) >= F.refill) {
+      // settle and write the finished rays together
+      if (unwritten) {
+        unwritten = false;
+        if (tr.settled(sc.tris, sc.tri_boxes, sc.obj_boxes, stack)) {
+          __stcs(q.hit + tr.st.get(stack, swrx::kRowUser).x, tr.st.get(stack, swrx::kRowHit));
+        } else {
+          tr.start_strict(stack);
           active = true;
+        }
+      }
+      idle = __ballot_sync(0xffffffffu, !active);
+      if (!exhausted) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(&ctrl->cursor[qp], (unsigned)__popc(idle));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= n) exhausted = true;
+        if (!active) {
+          const unsigned j = base + __popc(idle & lt);
+          if (j < n) {
+            const float4 o = __ldcs(q.o + j), d = __ldcs(q.d + j);
+            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack);
+            tr.st.set(stack, swrx::kRowUser, make_uint2(j, 0u));
+            active = true;
+          }
         }
       }
     }
@@ -449,9 +469,9 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tr.template step<kStats, kPostpone>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, &st)) {
-      __stcs(q.hit + ray, make_uint2(tr.hit.slot, __float_as_uint(tr.hit.t)));
+    if (active && tr.template step<kStats, kPostpone>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
       active = false;
+      unwritten = true;
     }
   }
   if (kStats) {
@@ -482,11 +502,12 @@ using swrx::kAdjMaxDepth;
 __global__ void __launch_bounds__(kTraceBlock)
     k_adjoint(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, const float* __restrict__ dl,
               float* __restrict__ g_alb, float* __restrict__ g_em) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const unsigned lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   const unsigned long long total = ctrl->total;
   swrx::Traversal tr;
+  tr.setup(stack);
   swrx::PathState st;
   uint32_t pixel = 0, sample = 0;
   swrx::AdjointTape tape;
@@ -519,6 +540,7 @@ __global__ void __launch_bounds__(kTraceBlock)
             st.v = 0;
             pend_slot = bits & 0x07FFFFFFu;
             pend_t = r0.w;
+            tr.no_hit(stack);  // the camera record's hit is settled
             tape.reset();
             tracing = false;
             active = true;
@@ -530,13 +552,13 @@ __global__ void __launch_bounds__(kTraceBlock)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, nullptr)) {
+    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
       tracing = false;
-      if (tr.hit.slot == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
+      if (tr.hit_slot(stack) == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
         active = false;
       } else {
-        pend_slot = tr.hit.slot;
-        pend_t = tr.hit.t;
+        pend_slot = tr.hit_slot(stack);
+        pend_t = tr.hit_t(stack);
       }
     }
     // lanes with a pending hit wait until F.batch of them (or every active lane) shade together
@@ -544,6 +566,11 @@ __global__ void __launch_bounds__(kTraceBlock)
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);
     if (waiting == 0u || ((unsigned)__popc(waiting) < F.batch && inflight != 0u)) continue;
     if (!active || tracing) continue;
+    if (!tr.settled(sc.tris, sc.tri_boxes, sc.obj_boxes, stack)) {
+      tr.start_strict(stack);
+      tracing = true;
+      continue;
+    }
     // shade the pending hit
     swrx::ShadeParams P;
     P.seed = F.seed;
@@ -561,7 +588,7 @@ __global__ void __launch_bounds__(kTraceBlock)
     // emitter (depth reached, Russian roulette, escape) carries no radiance and no gradient
     if (outcome == swrx::kContinue) {
       tape.push(pend_slot, c_before, av);
-      tr.init(st.o, st.d, stack + threadIdx.x, kTraceBlock);
+      tr.init(st.o, st.d, stack);
       tracing = true;
       continue;
     }
@@ -632,11 +659,12 @@ __device__ __forceinline__ f3 bd_get(const BdptArgs& B, uint32_t slot, uint32_t 
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_bdpt_paths(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, BdptArgs B) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const unsigned lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   const unsigned long long total = ctrl->total;
   swrx::Traversal tr;
+  tr.setup(stack);
   uint32_t pixel = 0, sample = 0, phase = kVision, i = 0, draws = 0, vfirst = 0, dv = 0, dl = 0;
   bool active = false, tracing = false, exhausted = false, vlight = false;
   f3 o = mk(0, 0, 0), d = mk(0, 0, 0), c = mk(1, 1, 1);
@@ -667,6 +695,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
             vfirst = i;
             hslot = bits & 0x07FFFFFFu;
             ht = r0.w;
+            tr.no_hit(stack);  // the camera record's hit is settled
             draws = 0;
             dv = dl = 0;
             vlight = false;
@@ -682,10 +711,10 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, nullptr)) {
+    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
       tracing = false;
-      hslot = tr.hit.slot;
-      ht = tr.hit.t;
+      hslot = tr.hit_slot(stack);
+      ht = tr.hit_t(stack);
     }
     // Lanes whose trace is finished wait until B.batch of them (or every active lane) can run
     // their stage code together, instead of running it for one or two lanes at a time.
@@ -693,6 +722,11 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);
     if (waiting == 0u || ((unsigned)__popc(waiting) < B.batch && inflight != 0u)) continue;
     if (!active || tracing) continue;
+    if (!tr.settled(sc.tris, sc.tri_boxes, sc.obj_boxes, stack)) {
+      tr.start_strict(stack);
+      tracing = true;
+      continue;
+    }
     const uint32_t gpix = F.pixel0 + pixel;
     const uint32_t q = pixel * F.spp + sample;
     // advance the sample until it needs a trace or is finished
@@ -740,7 +774,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
           }
           continue;
         }
-        tr.init(o, d, stack + threadIdx.x, kTraceBlock);
+        tr.init(o, d, stack);
         tracing = true;
       } else if (phase == kVisionDone) {
         if (vlight) {  // c is the throughput recorded at the last vision vertex
@@ -779,7 +813,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
         i = 1;
         if (B.lj > 1) {
           phase = kLight;
-          tr.init(o, d, stack + threadIdx.x, kTraceBlock);
+          tr.init(o, d, stack);
           tracing = true;
         } else {
           B.head[q] = make_uint4(vfirst, dv, dl, 0u);
@@ -799,11 +833,12 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_bdpt_connect(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, BdptArgs B) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const unsigned lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   const unsigned long long total = B.nsamp;
   swrx::Traversal tr;
+  tr.setup(stack);
   uint32_t q = 0, vi = 0, li = 0, dv = 0, dl = 0;
   bool active = false, tracing = false, exhausted = false, pending = false;
   f3 acc = mk(0.0f, 0.0f, 0.0f), dn = mk(0.0f, 0.0f, 0.0f);
@@ -838,14 +873,20 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, nullptr))
+    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
       tracing = false;
     const unsigned waiting = __ballot_sync(0xffffffffu, active && !tracing);
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);
     if (waiting == 0u || ((unsigned)__popc(waiting) < B.cbatch && inflight != 0u)) continue;
     if (!active || tracing) continue;
+    if (pending && !tr.settled(sc.tris, sc.tri_boxes, sc.obj_boxes, stack)) {
+      const f3 dd = swrx::vsub(bd_get(B, B.vj + li, 0, q), bd_get(B, vi, 0, q));
+      tr.start_occlusion_strict(swrx::vdot(dd, dd), stack);
+      tracing = true;
+      continue;
+    }
     if (pending) {  // the query of pair (vi, li) is answered
-      if (tr.hit.slot == 0xFFFFFFFFu) {  // not occluded
+      if (tr.hit_slot(stack) == 0xFFFFFFFFu) {  // not occluded
         const float cs = swrx::vdot(dn, bd_get(B, vi, 1, q));
         const f3 vc = bd_get(B, vi, 2, q), lc = bd_get(B, B.vj + li, 2, q);
         acc = swrx::vadd(acc, mk(__fmul_rn(__fmul_rn(vc.x, lc.x), cs), __fmul_rn(__fmul_rn(vc.y, lc.y), cs),
@@ -875,7 +916,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       const f3 dd = swrx::vsub(b, a);
       const float dist2 = swrx::vdot(dd, dd);
       dn = swrx::vnormalize(dd);
-      tr.init_occlusion(a, dn, dist2, stack + threadIdx.x, kTraceBlock);
+      tr.init_occlusion(a, dn, dist2, stack);
       tracing = true;
       pending = true;
       break;
@@ -1219,12 +1260,11 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   TraceKernel trace_kernel;
   const bool postpone = (o->flags & SWR_RENDER_POSTPONE) != 0;
   switch (o->trace_blocks) {
-    case 0:  // default: 9 blocks per SM (56 registers, no spills; measured faster than the
-             // compiler's own choice of 64 registers and 8 blocks)
     case 9:
       trace_kernel = postpone ? (count ? k_trace_dyn<true, 9, true> : k_trace_dyn<false, 9, true>)
                               : (count ? k_trace_dyn<true, 9, false> : k_trace_dyn<false, 9, false>);
       break;
+    case 0:  // default: 10 blocks per SM (48 registers, no spills)
     case 10:
       trace_kernel = postpone ? (count ? k_trace_dyn<true, 10, true> : k_trace_dyn<false, 10, true>)
                               : (count ? k_trace_dyn<true, 10, false> : k_trace_dyn<false, 10, false>);
@@ -1811,7 +1851,7 @@ int render_noalloc_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
   F.contrib = (float4*)(base + kNoAllocContribOffset);
 
   int trace_per_sm = 0;
-  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&trace_per_sm, k_trace_dyn<false, 0, false>,
+  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&trace_per_sm, k_trace_dyn<false, 10, false>,
                                                          kTraceBlock, 0));
   const unsigned trace_grid = (unsigned)(s->num_sms * std::max(trace_per_sm, 1));
   const unsigned shade_grid = (cap + 255) / 256;
@@ -1837,7 +1877,7 @@ int render_noalloc_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
       for (int c = 0; c < 8; ++c, ++k) {
         const int p = (int)(k & 1);
         k_shade<256><<<shade_grid, 256, 0, stream>>>(s->dev, F, ctrl, Q[p], Q[p ^ 1], p);
-        k_trace_dyn<false, 0, false><<<trace_grid, kTraceBlock, 0, stream>>>(s->dev, F, ctrl, Q[p ^ 1], p);
+        k_trace_dyn<false, 10, false><<<trace_grid, kTraceBlock, 0, stream>>>(s->dev, F, ctrl, Q[p ^ 1], p);
       }
       SWR_CUDA(cudaGetLastError());
       Ctrl h;

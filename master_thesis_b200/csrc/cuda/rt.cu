@@ -33,7 +33,7 @@ using swrx::f3;
 using swrx::mk;
 namespace rt = swrx::rt;
 
-constexpr int kBlock = 128;
+constexpr int kBlock = swrx::kTraceThreads;
 constexpr uint32_t kMiss = 0xFFFFFFFFu;
 constexpr uint32_t kMaxJumps = 1u << 16;
 constexpr uint32_t kMaxSpp = 1u << 24;
@@ -89,12 +89,13 @@ struct DefPayload {
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kBlock, kMinBlocks)
     k_rt_path(DevScene sc, RtFrame F, unsigned long long* __restrict__ cursor) {
-  __shared__ uint2 stack[swrx::kStackShared * kBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kBlock];
   __shared__ DefPayload defs;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
   const unsigned long long total = (unsigned long long)F.W * F.H;
   swrx::Traversal tr;
+  tr.setup(stack);
   rt::Payload cur;
   float def_eta = 0.0f;
   uint32_t pixel = 0, rng = 0, s = 0, i = 0, cull = 0, stage = kPrimary;
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
           cull = 0;
           fin = mk(0.0f, 0.0f, 0.0f);
           stage = kPrimary;
-          tr.init(o, d, stack + threadIdx.x, kBlock);
+          tr.init(o, d, stack);
           tracing = true;
           active = true;
         }
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       continue;
     }
     if (active && tracing &&
-        tr.step<false, false, swrx::kRuleRayQuery>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, nullptr))
+        tr.step<false, false, swrx::kRuleRayQuery>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
       tracing = false;
     // Lanes whose ray is finished wait until shade_batch of them (or every active lane) can shade
     // together: the shading code then runs once for many lanes instead of once per finished ray.
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);
     if (waiting == 0u || ((unsigned)__popc(waiting) < F.shade_batch && inflight != 0u)) continue;
     if (!active || tracing) continue;
-    const uint32_t hs = tr.hit.slot;
+    const uint32_t hs = tr.hit_slot(stack);
     if (stage == kPrimary) {
       // traceRay with back-face culling: up to four traces, each retry from the culled hit
       if (hs == kMiss) {
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       if (swrx::vdot(P.n, d) > 0.0f && cull < 3) {
         o = P.pos;
         ++cull;
-        tr.init(o, d, stack + threadIdx.x, kBlock);
+        tr.init(o, d, stack);
         tracing = true;
         continue;
       }
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
         col = swrx::vmul(col, mk(swrx::fmul(cur.color.x, cs), swrx::fmul(cur.color.y, cs),
                                  swrx::fmul(cur.color.z, cs)));
       }
-      tr.init(o, d, stack + threadIdx.x, kBlock);
+      tr.init(o, d, stack);
       tracing = true;
       stage = kJumpResult;
     }

@@ -108,7 +108,7 @@ int device_pack(swr_scene* s, const swr_scene_desc* d, const swr_build_opts* opt
   return SWR_OK;
 }
 
-constexpr int kTraceBlock = 128;
+constexpr int kTraceBlock = swrx::kTraceThreads;
 
 // albedo given per triangle id -> the per-slot array the kernels read
 __global__ void k_set_albedo(const uint32_t* __restrict__ slot_of, const float* __restrict__ by_id,
@@ -149,32 +149,50 @@ int device_input(const float* p, size_t bytes, cudaStream_t stream, void** tmp, 
 constexpr unsigned kRefill = 8;
 
 template <bool kStats, int kRule = swrx::kRuleReference>
-__global__ void __launch_bounds__(kTraceBlock)
+__global__ void __launch_bounds__(kTraceBlock, 10)
     k_trace_closest(DevScene sc, const float4* __restrict__ ro, const float4* __restrict__ rd,
                     uint64_t n, uint4* __restrict__ out, uint2* __restrict__ counts,
                     unsigned long long* __restrict__ cursor) {
-  __shared__ uint2 stack[swrx::kStackShared * kTraceBlock];
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
   swrx::Traversal tr;
+  tr.setup(stack);
   swrx::TraceStats st{0, 0};
   bool active = false, exhausted = false;
-  uint64_t ray = 0;
+  bool unwritten = false;  // the lane is idle and its finished ray (row kRowUser) is not written yet
   for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    if (!exhausted && (unsigned)__popc(idle) >= kRefill) {
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(cursor, (unsigned long long)__popc(idle));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= n) exhausted = true;
-      if (!active) {
-        const uint64_t j = base + (unsigned)__popc(idle & lt);
-        if (j < n) {
-          const float4 o = ro[j], d = rd[j];
-          tr.init(swrx::mk(o.x, o.y, o.z), swrx::mk(d.x, d.y, d.z), stack + threadIdx.x, kTraceBlock);
-          st = swrx::TraceStats{0, 0};
-          ray = j;
+    unsigned idle = __ballot_sync(0xffffffffu, !active);
+    if (exhausted ? idle == 0xffffffffu : (unsigned)__popc(idle) >= kRefill) {
+      // settle and write the finished rays together
+      if (unwritten) {
+        unwritten = false;
+        if (kRule == swrx::kRuleRayQuery || tr.settled(sc.tris, sc.tri_boxes, sc.obj_boxes, stack)) {
+          const swrx::Hit h = tr.result(sc.tris, stack);
+          const uint2 r = tr.st.get(stack, swrx::kRowUser);
+          const uint64_t ray = r.x | (uint64_t)r.y << 32;
+          out[ray] = make_uint4(h.id, h.obj, __float_as_uint(h.d2), __float_as_uint(h.t));
+          if (kStats) counts[ray] = make_uint2(st.nodes, st.tris);
+        } else {
+          tr.start_strict(stack);
           active = true;
+        }
+      }
+      idle = __ballot_sync(0xffffffffu, !active);
+      if (!exhausted) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(cursor, (unsigned long long)__popc(idle));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= n) exhausted = true;
+        if (!active) {
+          const uint64_t j = base + (unsigned)__popc(idle & lt);
+          if (j < n) {
+            const float4 o = ro[j], d = rd[j];
+            tr.init(swrx::mk(o.x, o.y, o.z), swrx::mk(d.x, d.y, d.z), stack);
+            st = swrx::TraceStats{0, 0};
+            tr.st.set(stack, swrx::kRowUser, make_uint2((uint32_t)j, (uint32_t)(j >> 32)));
+            active = true;
+          }
         }
       }
     }
@@ -182,11 +200,9 @@ __global__ void __launch_bounds__(kTraceBlock)
       if (exhausted) break;
       continue;
     }
-    if (active && tr.template step<kStats, false, kRule>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, &st)) {
-      const swrx::Hit h = tr.result(sc.tris);
-      out[ray] = make_uint4(h.id, h.obj, __float_as_uint(h.d2), __float_as_uint(h.t));
-      if (kStats) counts[ray] = make_uint2(st.nodes, st.tris);
+    if (active && tr.template step<kStats, false, kRule>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
       active = false;
+      unwritten = true;
     }
   }
 }

@@ -18,6 +18,8 @@
 #include <stdexcept>
 #include <thread>
 
+#include "../plane_grid.h"
+
 namespace swr {
 
 namespace {
@@ -538,21 +540,8 @@ WideBvh build_wide_bvh(const std::vector<PrimBox>& prims, const WideBvhOptions& 
     uint8_t qlo[3][8], qhi[3][8];
     std::memset(qlo, 255, sizeof(qlo));
     std::memset(qhi, 0, sizeof(qhi));
-    uint32_t ebyte[3];
-    double e[3];
-    for (int k = 0; k < 3; ++k) {
-      const double ext = (double)uhi[k] - (double)ulo[k];
-      int ex = -126;
-      if (ext > 0.0) {
-        int x;
-        std::frexp(ext / 255.0, &x);  // ext/255 = m * 2^x, m in [0.5, 1)
-        ex = x;
-        if (std::ldexp(1.0, ex - 1) >= ext / 255.0) ex = ex - 1;
-      }
-      ex = std::max(-126, std::min(127, ex));
-      ebyte[k] = (uint32_t)(ex + 127);
-      e[k] = std::ldexp(1.0, ex);
-    }
+    swrx::PlaneGrid grid[3];
+    for (int k = 0; k < 3; ++k) grid[k] = swrx::plane_grid(ulo[k], uhi[k]);
     uint32_t imask = 0;
     uint8_t meta[8] = {0};
     uint32_t tri_off = 0;
@@ -561,10 +550,8 @@ WideBvh build_wide_bvh(const std::vector<PrimBox>& prims, const WideBvhOptions& 
       const int32_t c = tk.child[s];
       if (c < 0) continue;
       for (int k = 0; k < 3; ++k) {
-        double lo = std::floor(((double)bn[c].lo[k] - (double)ulo[k]) / e[k]);
-        double hi = std::ceil(((double)bn[c].hi[k] - (double)ulo[k]) / e[k]);
-        qlo[k][s] = (uint8_t)std::max(0.0, std::min(255.0, lo));
-        qhi[k][s] = (uint8_t)std::max(0.0, std::min(255.0, hi));
+        qlo[k][s] = (uint8_t)swrx::plane_below(grid[k], bn[c].lo[k]);
+        qhi[k][s] = (uint8_t)swrx::plane_above(grid[k], bn[c].hi[k]);
       }
       if (tk.leaf_mask & (1u << s)) {
         // the leaf's primitives, left-first
@@ -587,10 +574,8 @@ WideBvh build_wide_bvh(const std::vector<PrimBox>& prims, const WideBvhOptions& 
         imask |= 1u << s;
       }
     }
-    put_f(w, 0, ulo[0]);
-    put_f(w, 1, ulo[1]);
-    put_f(w, 2, ulo[2]);
-    w[3] = ebyte[0] | (ebyte[1] << 8) | (ebyte[2] << 16) | (imask << 24);
+    for (int k = 0; k < 3; ++k) put_f(w, k, grid[k].origin);
+    w[3] = grid[0].ebyte | (grid[1].ebyte << 8) | (grid[2].ebyte << 16) | (imask << 24);
     w[4] = tk.child_base;
     w[5] = tk.tri_base;
     w[6] = meta[0] | (meta[1] << 8) | (meta[2] << 16) | ((uint32_t)meta[3] << 24);
