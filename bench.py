@@ -34,8 +34,8 @@ CONFIGS = {
     # name: scene parameters, image, spp, depth
     # wave_size: paths in flight, 2^27 measured best for this image by the autotuner (2^24..2^27
     # with refill 4-12 and shading blocks 256/512): the whole image's 132.7 M samples are in flight
-    # at once. The library's default of 2^23 bounds a scene's queue memory at 1.2 GB; 2^27 takes
-    # 19.3 GB
+    # at once. The library's default of 2^23 bounds a scene's queue memory at 0.94 GB; 2^27 takes
+    # 15.0 GB
     "c2": dict(kind="terrain", cells=1024, tile=16, spheres=64, subdiv=4, lights=4, W=1920, H=1080, spp=64,
                depth=8, seed=2024, microbench_rays=1 << 24, wave_size=1 << 27),
     "c1": dict(kind="cornell", W=256, H=256, spp=16, depth=5, seed=1),

@@ -68,7 +68,6 @@ struct BQueue {
   float4* o;  // origin | pixel (within the job)
   float4* d;  // direction | sample
   float4* c;  // throughput | job << 16 | i << 8 | v
-  float4* l;  // physical radiance so far
   uint2* hit;
 };
 
@@ -83,7 +82,15 @@ struct BArgs {
   unsigned long long* accum;    // [npix*3] fixed point
 };
 
+constexpr size_t kPathBytes = 3 * sizeof(float4) + sizeof(uint2);  // of one path in one queue
+
 __device__ __forceinline__ unsigned lane() { return threadIdx.x & 31u; }
+
+// pixel of a job's sample index (a job has fewer than 2^32 pixels); the 64-bit division only for
+// indices that need it
+__device__ __forceinline__ uint32_t div_spp(uint64_t local, uint32_t spp) {
+  return (local >> 32) ? (uint32_t)(local / spp) : (uint32_t)local / spp;
+}
 
 // index of the job whose [base, next base) range holds v (bases ascending, first is 0)
 __device__ __forceinline__ uint32_t find_job(const BJob* jobs, uint32_t n, uint64_t v, bool by_pixel) {
@@ -189,6 +196,8 @@ static unsigned bcamera_grid(int num_sms, uint64_t np) {
 }
 
 __device__ __forceinline__ void accumulate(unsigned long long* acc, float r, float g, float b) {
+  // nothing gathered (an emitter seen from behind): a zero adds nothing
+  if (((__float_as_uint(r) | __float_as_uint(g) | __float_as_uint(b)) << 1) == 0u) return;
   atomicAdd(acc + 0, (unsigned long long)__double2ll_rn((double)r * kFix));
   atomicAdd(acc + 1, (unsigned long long)__double2ll_rn((double)g * kFix));
   atomicAdd(acc + 2, (unsigned long long)__double2ll_rn((double)b * kFix));
@@ -197,7 +206,7 @@ __device__ __forceinline__ void accumulate(unsigned long long* acc, float r, flo
 // Shading round of the batch (as the single-scene k_shade): entries without a hit end at once; a
 // persistent grid's warps walk chunks of 32 entries, list the rest (entry, job) in their own
 // shared-memory lists and shade them 32 at a time.
-__global__ void __launch_bounds__(256) k_bshade(BArgs A, BCtrl* __restrict__ ctrl, BQueue in, BQueue out,
+__global__ void __launch_bounds__(256, 4) k_bshade(BArgs A, BCtrl* __restrict__ ctrl, BQueue in, BQueue out,
                                                 int parity) {
   __shared__ uint2 pending[8][64];
   const uint32_t n_in = ctrl->count[parity];
@@ -217,24 +226,12 @@ __global__ void __launch_bounds__(256) k_bshade(BArgs A, BCtrl* __restrict__ ctr
       bool has_hit = false;
       uint32_t job = 0;
       if (i < n_in) {
-        const uint2 h = in.hit[i];
-        const uint32_t meta = __float_as_uint(in.c[i].w);
-        job = meta >> 16;
-        if (h.x != kDead) {
-          has_hit = true;
-        } else {
-          const BJob& J = A.jobs[job];
-          if (J.mode != 0) {  // physical mode: the path ends with the radiance it gathered
-            const uint32_t pixel = __float_as_uint(in.o[i].w);
-            const float4 ql = in.l[i];
-            accumulate(A.accum + 3 * (J.pixel_base + pixel), ql.x, ql.y, ql.z);
-          }
-        }
+        has_hit = in.hit[i].x != kDead;  // else: the path left the scene having gathered nothing
       } else if (i < total) {
         const unsigned long long g = inj_base + (i - n_in);
         job = find_job(A.jobs, A.njobs, g, false);
         const BJob& J = A.jobs[job];
-        const uint64_t p = J.pixel_base + (g - J.sample_base) / J.spp;
+        const uint64_t p = J.pixel_base + div_spp(g - J.sample_base, J.spp);
         has_hit = __float_as_uint(A.cam[2 * p + 1].w) != kDead;  // else: a background pixel, nothing gathered
       }
       const unsigned m = __ballot_sync(0xffffffffu, has_hit);
@@ -253,32 +250,30 @@ __global__ void __launch_bounds__(256) k_bshade(BArgs A, BCtrl* __restrict__ ctr
         const uint2 w = list[npend + ln];
         const uint32_t e = w.x;
         job = w.y;
-        const BJob& J = A.jobs[job];
+        st.L = mk(0.0f, 0.0f, 0.0f);  // emitters end their path, so none has gathered anything yet
         if (e < n_in) {
           const float4 qo = in.o[e], qd = in.d[e], qc = in.c[e];
           const uint2 h = in.hit[e];
           pixel = __float_as_uint(qo.w);
           sample = __float_as_uint(qd.w);
           const uint32_t meta = __float_as_uint(qc.w);
+          job = meta >> 16;
           st.o = mk(qo.x, qo.y, qo.z);
           st.d = mk(qd.x, qd.y, qd.z);
           st.c = mk(qc.x, qc.y, qc.z);
           st.i = (meta >> 8) & 0xFFu;
           st.v = meta & 0xFFu;
-          const float4 ql = in.l[e];
-          st.L = mk(ql.x, ql.y, ql.z);
           slot = h.x;
           t = __uint_as_float(h.y);
         } else {
-          const unsigned long long g = inj_base + (e - n_in);
-          const uint64_t local = g - J.sample_base;
-          pixel = (uint32_t)(local / J.spp);
-          sample = (uint32_t)(local % J.spp);
+          const BJob& J = A.jobs[job];
+          const uint64_t local = inj_base + (e - n_in) - J.sample_base;
+          pixel = div_spp(local, J.spp);
+          sample = (uint32_t)(local - (uint64_t)pixel * J.spp);
           const uint64_t p = J.pixel_base + pixel;
           const float4 r0 = A.cam[2 * p], r1 = A.cam[2 * p + 1];
           const uint32_t bits = __float_as_uint(r1.w);
           st.c = mk(1.0f, 1.0f, 1.0f);
-          st.L = mk(0.0f, 0.0f, 0.0f);
           st.v = 0;
           st.o = mk(r0.x, r0.y, r0.z);
           st.d = mk(r1.x, r1.y, r1.z);
@@ -286,6 +281,7 @@ __global__ void __launch_bounds__(256) k_bshade(BArgs A, BCtrl* __restrict__ ctr
           slot = bits & 0x07FFFFFFu;
           t = r0.w;
         }
+        const BJob& J = A.jobs[job];
         const DevScene& sc = A.scenes[J.scene];
         swrx::ShadeParams P;
         P.seed = J.seed;
@@ -319,7 +315,6 @@ __global__ void __launch_bounds__(256) k_bshade(BArgs A, BCtrl* __restrict__ ctr
           out.o[j] = make_float4(st.o.x, st.o.y, st.o.z, __uint_as_float(pixel));
           out.d[j] = make_float4(st.d.x, st.d.y, st.d.z, __uint_as_float(sample));
           out.c[j] = make_float4(st.c.x, st.c.y, st.c.z, __uint_as_float((job << 16) | (st.i << 8) | st.v));
-          out.l[j] = make_float4(st.L.x, st.L.y, st.L.z, 0.0f);
         }
       }
     }
@@ -424,8 +419,8 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
         if (g < total) {
           J = &A.jobs[find_job(A.jobs, A.njobs, g, false)];
           const uint64_t local = g - J->sample_base;
-          pixel = (uint32_t)(local / J->spp);
-          sample = (uint32_t)(local % J->spp);
+          pixel = div_spp(local, J->spp);
+          sample = (uint32_t)(local - (uint64_t)pixel * J->spp);
           const uint64_t p = J->pixel_base + pixel;
           const float4 r0 = A.cam[2 * p], r1 = A.cam[2 * p + 1];
           const uint32_t bits = __float_as_uint(r1.w);
@@ -656,7 +651,7 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   cap = std::max<uint32_t>(32, (cap + 255u) & ~255u);
   const uint32_t refill = (bo && bo->refill) ? bo->refill : 8;
   if (refill > 32) return set_error(SWR_ERR_INVALID, "swr: refill must be 0..32");
-  if ((rc = ensure_bytes(&b->qbuf, b->qbytes, (size_t)cap * (4 * sizeof(float4) + sizeof(uint2)) * 2))) return rc;
+  if ((rc = ensure_bytes(&b->qbuf, b->qbytes, (size_t)cap * kPathBytes * 2))) return rc;
   if ((rc = ensure_bytes(&b->cam, b->cambytes, pixels * 2 * sizeof(float4)))) return rc;
   if ((rc = ensure_bytes(&b->accum, b->accbytes, pixels * 3 * sizeof(unsigned long long)))) return rc;
   if ((rc = ensure_bytes(&b->jobs, b->jobbytes, n * sizeof(BJob)))) return rc;
@@ -716,12 +711,11 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   const unsigned sgrid = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>((capw + 255) / 256, (uint64_t)num_sms * std::max(shade_per_sm, 1)));
   auto queues = [&](int h, BQueue* Qh) {
-    char* p = (char*)b->qbuf + (size_t)h * ((size_t)capw * (4 * sizeof(float4) + sizeof(uint2)) * 2);
+    char* p = (char*)b->qbuf + (size_t)h * ((size_t)capw * kPathBytes * 2);
     for (int k = 0; k < 2; ++k) {
       Qh[k].o = (float4*)p; p += (size_t)capw * sizeof(float4);
       Qh[k].d = (float4*)p; p += (size_t)capw * sizeof(float4);
       Qh[k].c = (float4*)p; p += (size_t)capw * sizeof(float4);
-      Qh[k].l = (float4*)p; p += (size_t)capw * sizeof(float4);
       Qh[k].hit = (uint2*)p; p += (size_t)capw * sizeof(uint2);
     }
   };

@@ -63,9 +63,9 @@ struct Queue {
   float4* o;  // o.xyz | pixel (chunk-local)
   float4* d;  // d.xyz | sample
   float4* c;  // throughput | (i << 8) | v
-  float4* l;  // physical: gathered radiance
   uint2* hit;  // slot | t
 };
+constexpr size_t kPathBytes = 3 * sizeof(float4) + sizeof(uint2);  // of one path in one queue
 
 struct Frame {
   float vi[16], pi[16];
@@ -82,8 +82,38 @@ struct Frame {
   uint32_t refill;   // idle lanes that trigger a refill in the bounce traversal
   uint32_t batch;    // adjoint: lanes with a finished trace that shade together
   float4* cam;       // [npix*2] per-pixel first hit: (o, t) (d, slot | i << 27)
-  float4* contrib;   // [npix*spp] per-sample radiance + flag
+  float4* contrib;   // [npix*spp] per-sample radiance + flag, written for lit samples (all of them
+                     // by the bidirectional tracer)
+  uint32_t* lit;     // [npix*lit_words] one bit per sample that reached a light; null: contrib is whole
+  uint32_t lit_words;  // words per pixel
+  uint32_t div_mul, div_shift;  // division by spp (div_spp)
 };
+
+// Sample index of a chunk -> pixel of the chunk, without a division: the host gives the multiplier
+// ceil(2^(31+l) / spp) with l = ceil(log2 spp), exact for indices below 2^31 (a chunk holds at most
+// 2^27 samples, or one pixel, whose quotient is 0: multiplier 0). Two 64-bit divisions per injected
+// sample were a fifth of the shading kernel's instructions.
+constexpr uint32_t kDivOne = 0xFFu;
+__device__ __forceinline__ uint32_t div_spp(const Frame& F, uint32_t g) {
+  return F.div_shift == kDivOne ? g : __umulhi(g, F.div_mul) >> F.div_shift;
+}
+void set_div_spp(Frame& F, uint64_t chunk_pixels) {
+  if (chunk_pixels <= 1) {
+    F.div_mul = F.div_shift = 0;
+  } else if (F.spp == 1) {
+    F.div_mul = 0;
+    F.div_shift = kDivOne;
+  } else {
+    uint32_t l = 1;
+    while ((1ull << l) < F.spp) ++l;
+    F.div_mul = (uint32_t)(((1ull << (31 + l)) + F.spp - 1) / F.spp);
+    F.div_shift = l - 1;
+  }
+}
+
+// Words of lit bits per pixel, and from how many on the host clears them instead of k_camera.
+constexpr uint32_t lit_words_of(uint32_t spp) { return spp / 32u + (spp % 32u ? 1u : 0u); }
+constexpr uint32_t kLitClearedByCamera = 32;
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
@@ -156,6 +186,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
       if (done) {
         F.cam[2 * (size_t)k] = rec0;
         F.cam[2 * (size_t)k + 1] = rec1;
+        if (F.lit && F.lit_words <= kLitClearedByCamera)
+          for (uint32_t w = 0; w < F.lit_words; ++w) F.lit[(size_t)k * F.lit_words + w] = 0u;
         active = false;
       }
     }
@@ -189,6 +221,7 @@ __device__ __forceinline__ ShadeEntry load_entry(const Frame& F, const Queue& in
   ShadeEntry e;
   e.slot = kDeadSlot;
   e.t = 0.0f;
+  e.st.L = mk(0.0f, 0.0f, 0.0f);  // emitters end their path, so none has gathered anything yet
   if (i < n_in) {
     const float4 qo = __ldcs(in.o + i), qd = __ldcs(in.d + i), qc = __ldcs(in.c + i);
     const uint2 h = __ldcs(in.hit + i);
@@ -200,22 +233,15 @@ __device__ __forceinline__ ShadeEntry load_entry(const Frame& F, const Queue& in
     e.st.c = mk(qc.x, qc.y, qc.z);
     e.st.i = (meta >> 8) & 0xFFu;
     e.st.v = meta & 0xFFu;
-    if (F.mode == 1) {
-      const float4 ql = __ldcs(in.l + i);
-      e.st.L = mk(ql.x, ql.y, ql.z);
-    } else {
-      e.st.L = mk(0, 0, 0);
-    }
     e.slot = h.x;
     e.t = __uint_as_float(h.y);
   } else {
-    const unsigned long long g = inj_base + (i - n_in);
-    e.pixel = (uint32_t)(g / F.spp);
-    e.sample = (uint32_t)(g % F.spp);
+    const uint32_t g = (uint32_t)inj_base + (i - n_in);
+    e.pixel = div_spp(F, g);
+    e.sample = g - e.pixel * F.spp;
     const float4 r0 = F.cam[2 * (size_t)e.pixel], r1 = F.cam[2 * (size_t)e.pixel + 1];
     const uint32_t bits = __float_as_uint(r1.w);
     e.st.c = mk(1.0f, 1.0f, 1.0f);
-    e.st.L = mk(0.0f, 0.0f, 0.0f);
     e.st.v = 0;
     e.st.o = mk(r0.x, r0.y, r0.z);
     e.st.d = mk(r1.x, r1.y, r1.z);
@@ -230,7 +256,10 @@ __device__ __forceinline__ ShadeEntry load_entry(const Frame& F, const Queue& in
 
 // Shading round: entries [0, n_in) are the traced paths of the previous round, [n_in, n_in +
 // n_inj) new camera samples. An entry without a hit (a ray that left the scene, a camera sample
-// of a background pixel) ends dark at once. The grid is persistent: each warp walks chunks of 32
+// of a background pixel) ends dark, and a dark end leaves no trace: only a sample that reaches a
+// light writes its contribution slot and sets its bit in F.lit, so nothing but the hit word of a
+// missed entry is read (before, its pixel and sample words and a 16-byte zero: 80 bytes of DRAM
+// sectors for each of the terrain image's 130 M dark samples). The grid is persistent: each warp walks chunks of 32
 // entries, lists the entries with a hit in its own shared-memory list and shades them 32 at a
 // time, so that the long shading code (Philox, double-precision trigonometry and normalisation)
 // runs on full warps although most bounce rays miss, and no warp waits at a block barrier or
@@ -253,7 +282,8 @@ __global__ void __launch_bounds__(kBlock)
   // the hit word of entry i (the traced slot, or the camera record's slot bits), kDeadSlot for none
   auto hit_word = [&](uint64_t i) -> uint32_t {
     if (i < n_in) return in.hit[i].x;
-    if (i < total) return __float_as_uint(F.cam[2 * (size_t)((inj_base + (i - n_in)) / F.spp) + 1].w);
+    if (i < total)
+      return __float_as_uint(F.cam[2 * (size_t)div_spp(F, (uint32_t)inj_base + (uint32_t)(i - n_in)) + 1].w);
     return kDeadSlot;
   };
   uint64_t base = (uint64_t)blockIdx.x * kBlock + (threadIdx.x & ~31u);
@@ -261,31 +291,9 @@ __global__ void __launch_bounds__(kBlock)
   for (;; base += stride) {
     const bool more = base < total;
     if (more) {
-      // entries without a hit: their dark end; the rest: listed
+      // entries with a hit are listed; the others end dark
       const uint64_t i = base + lane;
-      bool has_hit = false;
-      if (i < n_in) {
-        if (word != kDeadSlot) {
-          has_hit = true;
-        } else {
-          const uint32_t pixel = __float_as_uint(__ldcs(&in.o[i].w));
-          const uint32_t sample = __float_as_uint(__ldcs(&in.d[i].w));
-          float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (F.mode == 1) {
-            const float4 ql = __ldcs(in.l + i);
-            r = make_float4(ql.x, ql.y, ql.z, 1.0f);
-          }
-          __stcs(F.contrib + (size_t)pixel * F.spp + sample, r);
-        }
-      } else if (i < total) {
-        if (word != kDeadSlot) {
-          has_hit = true;
-        } else {
-          const unsigned long long g = inj_base + (i - n_in);
-          const float4 r = (F.mode == 1) ? make_float4(0.0f, 0.0f, 0.0f, 1.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          __stcs(F.contrib + (size_t)(g / F.spp) * F.spp + (uint32_t)(g % F.spp), r);
-        }
-      }
+      const bool has_hit = i < total && word != kDeadSlot;
       const unsigned m = __ballot_sync(0xffffffffu, has_hit);
       if (has_hit) list[npend + __popc(m & lt)] = (uint32_t)i;
       npend += (uint32_t)__popc(m);
@@ -312,14 +320,13 @@ __global__ void __launch_bounds__(kBlock)
         const uint32_t outcome = swrx::shade_vertex(sc.tris, sc.shade, sc.mats, sc.albedo, e.slot, e.t, P, e.st);
         if (outcome == swrx::kContinue) {
           live = true;
-        } else {
-          float4 r;
-          if (F.mode == 0)
-            r = (outcome == swrx::kEndLight) ? make_float4(e.st.c.x, e.st.c.y, e.st.c.z, 1.0f)
-                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          else
-            r = make_float4(e.st.L.x, e.st.L.y, e.st.L.z, 1.0f);
-          __stcs(F.contrib + (size_t)e.pixel * F.spp + e.sample, r);
+        } else if (outcome == swrx::kEndLight) {
+          const f3 r = F.mode == 0 ? e.st.c : e.st.L;
+          // (an emitter seen from behind, physical mode: a zero adds nothing)
+          if (F.mode == 0 || ((__float_as_uint(r.x) | __float_as_uint(r.y) | __float_as_uint(r.z)) << 1) != 0u) {
+            __stcs(F.contrib + (size_t)e.pixel * F.spp + e.sample, make_float4(r.x, r.y, r.z, 1.0f));
+            atomicOr(F.lit + (size_t)e.pixel * F.lit_words + (e.sample >> 5), 1u << (e.sample & 31u));
+          }
         }
       }
       __syncwarp();  // the list slots just read may be refilled by the next chunk
@@ -335,7 +342,6 @@ __global__ void __launch_bounds__(kBlock)
           __stcs(out.o + j, make_float4(e.st.o.x, e.st.o.y, e.st.o.z, __uint_as_float(e.pixel)));
           __stcs(out.d + j, make_float4(e.st.d.x, e.st.d.y, e.st.d.z, __uint_as_float(e.sample)));
           __stcs(out.c + j, make_float4(e.st.c.x, e.st.c.y, e.st.c.z, __uint_as_float((e.st.i << 8) | e.st.v)));
-          if (F.mode == 1) __stcs(out.l + j, make_float4(e.st.L.x, e.st.L.y, e.st.L.z, 0.0f));
         }
       }
     }
@@ -527,8 +533,8 @@ __global__ void __launch_bounds__(kTraceBlock)
       if (!active) {
         const unsigned long long g = base + __popc(idle & lt);
         if (g < total) {
-          pixel = (uint32_t)(g / F.spp);
-          sample = (uint32_t)(g % F.spp);
+          pixel = div_spp(F, (uint32_t)g);
+          sample = (uint32_t)g - pixel * F.spp;
           const float4 r0 = F.cam[2 * (size_t)pixel], r1 = F.cam[2 * (size_t)pixel + 1];
           const uint32_t bits = __float_as_uint(r1.w);
           if (bits != kDeadSlot) {
@@ -681,8 +687,8 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (!active) {
         const unsigned long long g = base + __popc(idle & lt);
         if (g < total) {
-          pixel = (uint32_t)(g / F.spp);
-          sample = (uint32_t)(g % F.spp);
+          pixel = div_spp(F, (uint32_t)g);
+          sample = (uint32_t)g - pixel * F.spp;
           const float4 r0 = F.cam[2 * (size_t)pixel], r1 = F.cam[2 * (size_t)pixel + 1];
           const uint32_t bits = __float_as_uint(r1.w);
           if (bits == kDeadSlot) {  // no front hit within visionJumpCount: the sample adds nothing
@@ -897,7 +903,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     }
     for (;;) {
       if (vi >= dv) {
-        const uint32_t pixel = q / F.spp, sample = q % F.spp;
+        const uint32_t pixel = div_spp(F, q), sample = q - pixel * F.spp;
         const f3 r = swrx::vscale(inv_md, acc);
         F.contrib[(size_t)pixel * F.spp + sample] = make_float4(r.x, r.y, r.z, 1.0f);
         active = false;
@@ -924,11 +930,19 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
   }
 }
 
+// Slots of a chunk that samples_out wants whole: what a dark sample reports.
+__global__ void k_dark_samples(float4* __restrict__ contrib, uint64_t n, float flag) {
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
+    __stcs(contrib + k, make_float4(0.0f, 0.0f, 0.0f, flag));
+}
+
 // Per-pixel sum of the sample slots in sample order (path_tracer.cpp:28-37), 256 pixels per block.
-// A warp takes 32 consecutive pixels and loads their slots 8 samples at a time with coalesced loads
-// (each load instruction reads whole 128-byte lines) into a shared-memory tile padded to 9 slots
-// per pixel (conflict-free reads); each lane then adds its pixel's slots in sample order, as the
-// reference's renderPixel does.
+// A warp takes 32 consecutive pixels and 8 samples of each at a time. With F.lit only the slots of
+// lit samples are read, and groups without one are passed over: what is left of the terrain image's
+// 2.1 GB of slots is their few lit ones. The loads are coalesced (neighbouring lanes read
+// neighbouring slots of a pixel) into a shared-memory tile padded to 9 slots per pixel
+// (conflict-free reads); each lane then adds its pixel's slots in sample order, as the reference's
+// renderPixel does.
 __global__ void __launch_bounds__(256) k_resolve(Frame F, float* __restrict__ img) {
   __shared__ float4 tile[8][32 * 9];
   const uint32_t w = threadIdx.x >> 5, lane = lane_id();
@@ -938,25 +952,33 @@ __global__ void __launch_bounds__(256) k_resolve(Frame F, float* __restrict__ im
   const uint32_t spp = F.spp;
   float4* t = tile[w];
   float r = 0.0f, g = 0.0f, b = 0.0f;
-  for (uint32_t s0 = 0; s0 < spp; s0 += 8) {
-    const uint32_t ns = (spp - s0) < 8 ? (spp - s0) : 8;
+  const uint32_t words = lit_words_of(spp);
+  for (uint32_t k = 0; k < words; ++k) {
+    uint32_t bits = lane < np ? 0xFFFFFFFFu : 0u;
+    if (F.lit && lane < np) bits = F.lit[(size_t)(p0 + lane) * words + k];
+    if (!__any_sync(0xffffffffu, bits != 0u)) continue;
+    const uint32_t left = spp - 32u * k;  // samples from this word on
+    if (left < 32u) bits &= (1u << left) - 1u;
+    for (uint32_t s0 = 0; s0 < 32u && s0 < left; s0 += 8) {
+      const uint32_t mine = (bits >> s0) & 0xFFu;
+      if (!__any_sync(0xffffffffu, mine != 0u)) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t e = lane + 32u * j, pe = e >> 3, se = e & 7u;
-      if (pe < np && se < ns) t[pe * 9 + se] = __ldcs(F.contrib + (size_t)(p0 + pe) * spp + s0 + se);
-    }
-    __syncwarp();
-    if (lane < np) {
-      for (uint32_t k = 0; k < ns; ++k) {
-        const float4 v = t[lane * 9 + k];
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t e = lane + 32u * j, pe = e >> 3, se = e & 7u;
+        const uint32_t theirs = __shfl_sync(0xffffffffu, mine, pe);
+        if ((theirs >> se) & 1u) t[pe * 9 + se] = __ldcs(F.contrib + (size_t)(p0 + pe) * spp + 32u * k + s0 + se);
+      }
+      __syncwarp();
+      for (uint32_t m = mine; m; m &= m - 1u) {
+        const float4 v = t[lane * 9 + __ffs(m) - 1];
         if (v.w != 0.0f) {
           r = __fadd_rn(r, v.x);
           g = __fadd_rn(g, v.y);
           b = __fadd_rn(b, v.z);
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
   }
   if (lane >= np) return;
   // reference: finalColor *= 2.0f * M_PI * (1.0f / float(spp)), scalar and products in double
@@ -969,10 +991,11 @@ __global__ void __launch_bounds__(256) k_resolve(Frame F, float* __restrict__ im
 }
 
 struct Workspace {
-  size_t qbytes = 0, cam_px = 0, contrib_n = 0, stage_n = 0, bd_vtx_n = 0, bd_head_n = 0;
+  size_t qbytes = 0, cam_px = 0, contrib_n = 0, lit_n = 0, stage_n = 0, bd_vtx_n = 0, bd_head_n = 0;
   void* qbuf = nullptr;
   void* cam = nullptr;
   void* contrib = nullptr;
+  void* lit = nullptr;
   void* stage = nullptr;  // device image for callers that pass a host output buffer
   void* bd_vtx = nullptr;   // bidirectional tracer: per-sample vertex tables
   void* bd_head = nullptr;  // bidirectional tracer: per-sample vertex counts
@@ -1166,6 +1189,20 @@ static int image_part(const swr_render_opts* o, bool allow_samples, bool allow_p
   return SWR_OK;
 }
 
+// What a chunk's samples start from: no lit bits (k_camera clears a pixel's few words itself) and,
+// when the caller takes the slots whole, dark slots.
+static int clear_samples(const swr_scene* s, const Frame& F, bool want_samples, cudaStream_t st) {
+  if (F.lit_words > kLitClearedByCamera)
+    SWR_CUDA(cudaMemsetAsync(F.lit, 0, (size_t)F.npix * F.lit_words * sizeof(uint32_t), st));
+  if (want_samples) {
+    const uint64_t n = (uint64_t)F.npix * F.spp;
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)s->num_sms * 8);
+    k_dark_samples<<<grid, 256, 0, st>>>(F.contrib, n, F.mode == 1 ? 1.0f : 0.0f);
+    SWR_CUDA(cudaGetLastError());
+  }
+  return SWR_OK;
+}
+
 int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, float* rgb_out,
                 float* samples_out, void* stream_, swr_render_profile* prof) {
   if (!s || !cam || !o || !rgb_out) return set_error(SWR_ERR_INVALID, "swr: null argument");
@@ -1202,10 +1239,11 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   uint32_t cap = o->wave_size ? o->wave_size : (1u << 23);
   cap = (uint32_t)std::min<uint64_t>(cap, px_per_chunk * o->spp);
   cap = std::max<uint32_t>(32, (cap + 255u) & ~255u);
-  const size_t qbytes = (size_t)cap * (4 * sizeof(float4) + sizeof(uint2)) * 2;
+  const size_t qbytes = (size_t)cap * kPathBytes * 2;
   if ((rc = ensure(&ws->qbuf, ws->qbytes, qbytes, 1))) return rc;
   if ((rc = ensure(&ws->cam, ws->cam_px, px_per_chunk, 2 * sizeof(float4)))) return rc;
   if ((rc = ensure(&ws->contrib, ws->contrib_n, px_per_chunk * o->spp, sizeof(float4)))) return rc;
+  if ((rc = ensure(&ws->lit, ws->lit_n, px_per_chunk * lit_words_of(o->spp), sizeof(uint32_t)))) return rc;
   if (!ws->ctrl) {
     SWR_CUDA(cudaMalloc(&ws->ctrl, 4 * sizeof(Ctrl)));
     SWR_CUDA(cudaMallocHost(&ws->host_ctrl, 4 * sizeof(Ctrl)));
@@ -1218,7 +1256,6 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       Q[p].o = (float4*)b; b += (size_t)cap * sizeof(float4);
       Q[p].d = (float4*)b; b += (size_t)cap * sizeof(float4);
       Q[p].c = (float4*)b; b += (size_t)cap * sizeof(float4);
-      Q[p].l = (float4*)b; b += (size_t)cap * sizeof(float4);
       Q[p].hit = (uint2*)b; b += (size_t)cap * sizeof(uint2);
     }
   }
@@ -1254,6 +1291,9 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   F.capacity = cap;
   F.cam = (float4*)ws->cam;
   F.contrib = (float4*)ws->contrib;
+  F.lit = (uint32_t*)ws->lit;
+  F.lit_words = lit_words_of(o->spp);
+  set_div_spp(F, px_per_chunk);
 
   using TraceKernel = void (*)(DevScene, Frame, Ctrl*, Queue, int);
   const bool static_fetch = (o->flags & SWR_RENDER_STATIC_FETCH) != 0;
@@ -1285,12 +1325,11 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   auto launch_wave = [&](int h, cudaStream_t st, uint64_t p0, uint64_t off, uint32_t n, uint32_t capw) -> int {
     Queue Qh[2];
     {
-      char* b = (char*)ws->qbuf + (size_t)h * ((size_t)capw * (4 * sizeof(float4) + sizeof(uint2)) * 2);
+      char* b = (char*)ws->qbuf + (size_t)h * ((size_t)capw * kPathBytes * 2);
       for (int q = 0; q < 2; ++q) {
         Qh[q].o = (float4*)b; b += (size_t)capw * sizeof(float4);
         Qh[q].d = (float4*)b; b += (size_t)capw * sizeof(float4);
         Qh[q].c = (float4*)b; b += (size_t)capw * sizeof(float4);
-        Qh[q].l = (float4*)b; b += (size_t)capw * sizeof(float4);
         Qh[q].hit = (uint2*)b; b += (size_t)capw * sizeof(uint2);
       }
     }
@@ -1300,6 +1339,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     Fh.npix = n;
     Fh.cam = F.cam + 2 * off;
     Fh.contrib = F.contrib + off * o->spp;
+    Fh.lit = F.lit + off * F.lit_words;
     Fh.capacity = capw;
     const uint64_t total = (uint64_t)n * o->spp;
     // every path ends within max_depth rounds of its injection and each round injects up to the
@@ -1314,6 +1354,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     ws->host_ctrl[h] = init;
     SWR_CUDA(cudaMemcpyAsync(ctrl, ws->host_ctrl + h, sizeof(Ctrl), cudaMemcpyHostToDevice, st));
     P.h2d_bytes += sizeof(Ctrl);
+    if ((rc = clear_samples(s, Fh, want_samples, st))) return rc;
     k_camera<<<camera_grid(s, n), kTraceBlock, 0, st>>>(s->dev, Fh, ctrl);
     SWR_CUDA(cudaGetLastError());
     // the shading and traversal kernels read the first pixel from the control block, so their
@@ -1429,6 +1470,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       *ws->host_ctrl = init;
       SWR_CUDA(cudaMemcpyAsync(ws->ctrl, ws->host_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, stream));
       P.h2d_bytes += sizeof(Ctrl);
+      if ((rc = clear_samples(s, F, want_samples, stream))) return rc;
       SWR_CUDA(timer.begin(stream, kTimeCamera));
       k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl);
       SWR_CUDA(timer.end(stream));
@@ -1511,6 +1553,7 @@ void free_workspace(swr_scene* s) {
   if (ws->qbuf) cudaFree(ws->qbuf);
   if (ws->cam) cudaFree(ws->cam);
   if (ws->contrib) cudaFree(ws->contrib);
+  if (ws->lit) cudaFree(ws->lit);
   if (ws->stage) cudaFree(ws->stage);
   if (ws->bd_vtx) cudaFree(ws->bd_vtx);
   if (ws->bd_head) cudaFree(ws->bd_head);
@@ -1577,6 +1620,7 @@ int render_adjoint_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
   F.refill = o->refill ? o->refill : 8;
   F.batch = o->shade_batch ? o->shade_batch : swrx::kAdjointBatch;
   F.cam = (float4*)ws->cam;
+  set_div_spp(F, px_per_chunk);
   int per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint, kTraceBlock, 0));
   const unsigned grid = (unsigned)(s->num_sms * std::max(per_sm, 1));
@@ -1685,6 +1729,7 @@ int render_bdpt_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts*
   F.refill = o->refill ? o->refill : 4;
   F.cam = (float4*)ws->cam;
   F.contrib = (float4*)ws->contrib;
+  set_div_spp(F, px_per_chunk);
   BdptArgs B;
   B.vj = o->max_depth;
   B.lj = b->light_jumps;
@@ -1746,11 +1791,14 @@ constexpr size_t kNoAllocBytes = 64ull << 20;           // 64 MiB of device scra
 constexpr uint32_t kNoAllocCap = 1u << 16;              // paths in flight
 constexpr uint64_t kNoAllocChunkSamples = 1ull << 21;   // samples per chunk
 constexpr uint64_t kNoAllocChunkPixels = 1ull << 18;    // pixels per chunk
-constexpr size_t kNoAllocQueueBytes = (size_t)kNoAllocCap * (4 * sizeof(float4) + sizeof(uint2));
+constexpr size_t kNoAllocQueueBytes = (size_t)kNoAllocCap * kPathBytes;
 constexpr size_t kNoAllocCamOffset = 256 + 2 * kNoAllocQueueBytes;  // the control block takes the first 256 bytes
 static_assert(sizeof(Ctrl) <= 256, "the allocation-free render keeps its control block in 256 bytes");
 constexpr size_t kNoAllocContribOffset = kNoAllocCamOffset + kNoAllocChunkPixels * 2 * sizeof(float4);
-static_assert(kNoAllocContribOffset + kNoAllocChunkSamples * sizeof(float4) <= kNoAllocBytes,
+// lit bits: a word per pixel plus one per 32 samples bounds them
+constexpr size_t kNoAllocLitOffset = kNoAllocContribOffset + kNoAllocChunkSamples * sizeof(float4);
+constexpr size_t kNoAllocLitWords = kNoAllocChunkPixels + kNoAllocChunkSamples / 32;
+static_assert(kNoAllocLitOffset + kNoAllocLitWords * sizeof(uint32_t) <= kNoAllocBytes,
               "no-allocation scratch layout exceeds its array");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1825,7 +1873,6 @@ int render_noalloc_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
       Q[p].o = (float4*)b; b += (size_t)kNoAllocCap * sizeof(float4);
       Q[p].d = (float4*)b; b += (size_t)kNoAllocCap * sizeof(float4);
       Q[p].c = (float4*)b; b += (size_t)kNoAllocCap * sizeof(float4);
-      Q[p].l = (float4*)b; b += (size_t)kNoAllocCap * sizeof(float4);
       Q[p].hit = (uint2*)b; b += (size_t)kNoAllocCap * sizeof(uint2);
     }
   }
@@ -1849,6 +1896,9 @@ int render_noalloc_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
   F.refill = o->refill ? o->refill : 8;
   F.cam = (float4*)(base + kNoAllocCamOffset);
   F.contrib = (float4*)(base + kNoAllocContribOffset);
+  F.lit = (uint32_t*)(base + kNoAllocLitOffset);
+  F.lit_words = lit_words_of(o->spp);
+  set_div_spp(F, px_per_chunk);
 
   int trace_per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&trace_per_sm, k_trace_dyn<false, 10, false>,
@@ -1868,6 +1918,7 @@ int render_noalloc_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
     init.pixel0 = (uint32_t)p0;
     // pageable source: the copy has been taken when the call returns
     SWR_CUDA(cudaMemcpyAsync(ctrl, &init, sizeof(Ctrl), cudaMemcpyHostToDevice, stream));
+    if ((rc = clear_samples(s, F, want_samples, stream))) return rc;
     k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ctrl);
     SWR_CUDA(cudaGetLastError());
     uint64_t k = 0;
