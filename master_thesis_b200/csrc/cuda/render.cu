@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(kTraceBlock)
 // the queue with one atomic and the idle lanes start them. This keeps lanes busy while the
 // slowest ray of a batch is still walking the tree.
 // kMinBlocks > 0 caps the register budget so that many blocks fit on one SM.
-template <bool kStats, int kMinBlocks, bool kPostpone>
+template <bool kStats, int kMinBlocks, bool kPostpone, bool kTriLoop = false>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_trace_dyn(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tr.template step<kStats, kPostpone>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
+    if (active && tr.template step<kStats, kPostpone, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
       active = false;
       unwritten = true;
     }
@@ -505,6 +505,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
 // as in the bounce traversal), and the traversal itself is the resumable Traversal.
 using swrx::kAdjMaxDepth;
 
+template <bool kTriLoop>
 __global__ void __launch_bounds__(kTraceBlock)
     k_adjoint(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, const float* __restrict__ dl,
               float* __restrict__ g_alb, float* __restrict__ g_em) {
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(kTraceBlock)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
+    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
       tracing = false;
       if (tr.hit_slot(stack) == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
         active = false;
@@ -662,7 +663,7 @@ __device__ __forceinline__ f3 bd_get(const BdptArgs& B, uint32_t slot, uint32_t 
   return mk(v.x, v.y, v.z);
 }
 
-template <int kMinBlocks>
+template <int kMinBlocks, bool kTriLoop>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_bdpt_paths(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, BdptArgs B) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
@@ -717,7 +718,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
+    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
       tracing = false;
       hslot = tr.hit_slot(stack);
       ht = tr.hit_t(stack);
@@ -836,7 +837,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
 // the two points lifted by 0.01 along their normals; an unoccluded pair adds
 // (vision throughput * light throughput) * cos at the vision vertex. The sum, in that order, is
 // divided by maxDepth.
-template <int kMinBlocks>
+template <int kMinBlocks, bool kTriLoop>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_bdpt_connect(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, BdptArgs B) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
@@ -879,7 +880,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
+    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
       tracing = false;
     const unsigned waiting = __ballot_sync(0xffffffffu, active && !tracing);
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);
@@ -1308,6 +1309,8 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     case 10:
       trace_kernel = postpone ? (count ? k_trace_dyn<true, 10, true> : k_trace_dyn<false, 10, true>)
                               : (count ? k_trace_dyn<true, 10, false> : k_trace_dyn<false, 10, false>);
+      if (!postpone && s->dev.num_tris <= swrx::kFewTriangles)
+        trace_kernel = count ? k_trace_dyn<true, 10, false, true> : k_trace_dyn<false, 10, false, true>;
       break;
     default: return set_error(SWR_ERR_INVALID, "swr: trace_blocks must be 0, 9 or 10");
   }
@@ -1622,7 +1625,8 @@ int render_adjoint_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
   F.cam = (float4*)ws->cam;
   set_div_spp(F, px_per_chunk);
   int per_sm = 0;
-  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint, kTraceBlock, 0));
+  auto kern = s->dev.num_tris <= swrx::kFewTriangles ? k_adjoint<true> : k_adjoint<false>;
+  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));
   const unsigned grid = (unsigned)(s->num_sms * std::max(per_sm, 1));
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ms_out) {
@@ -1641,7 +1645,7 @@ int render_adjoint_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
     *ws->host_ctrl = init;
     SWR_CUDA(cudaMemcpyAsync(ws->ctrl, ws->host_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, stream));
     k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl);
-    k_adjoint<<<grid, kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl, dl, g_alb, g_em);
+    kern<<<grid, kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl, dl, g_alb, g_em);
     SWR_CUDA(cudaGetLastError());
   }
   if (ms_out) {
@@ -1738,11 +1742,12 @@ int render_bdpt_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts*
   B.cbatch = ((b->shade_batch >> 8) & 0xFFu) ? ((b->shade_batch >> 8) & 0xFFu) : kConnectBatch;
   B.vtx = (float4*)ws->bd_vtx;
   B.head = (uint4*)ws->bd_head;
-  auto kern = k_bdpt_paths<0>;
-  auto kconn = k_bdpt_connect<0>;
-  if (b->blocks_per_sm == 5) kern = k_bdpt_paths<5>, kconn = k_bdpt_connect<5>;
-  else if (b->blocks_per_sm == 6) kern = k_bdpt_paths<6>, kconn = k_bdpt_connect<6>;
-  else if (b->blocks_per_sm == 8) kern = k_bdpt_paths<8>, kconn = k_bdpt_connect<8>;
+  const bool few = s->dev.num_tris <= swrx::kFewTriangles;
+  auto kern = few ? k_bdpt_paths<0, true> : k_bdpt_paths<0, false>;
+  auto kconn = few ? k_bdpt_connect<0, true> : k_bdpt_connect<0, false>;
+  if (b->blocks_per_sm == 5) kern = k_bdpt_paths<5, false>, kconn = k_bdpt_connect<5, false>;
+  else if (b->blocks_per_sm == 6) kern = k_bdpt_paths<6, false>, kconn = k_bdpt_connect<6, false>;
+  else if (b->blocks_per_sm == 8) kern = k_bdpt_paths<8, false>, kconn = k_bdpt_connect<8, false>;
   int per_sm = 0, per_sm_c = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, kconn, kTraceBlock, 0));

@@ -86,7 +86,7 @@ struct DefPayload {
 };
 
 // kMinBlocks: resident blocks per SM the register budget targets (0 = the compiler's choice)
-template <int kMinBlocks>
+template <int kMinBlocks, bool kTriLoop>
 __global__ void __launch_bounds__(kBlock, kMinBlocks)
     k_rt_path(DevScene sc, RtFrame F, unsigned long long* __restrict__ cursor) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kBlock];
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       continue;
     }
     if (active && tracing &&
-        tr.step<false, false, swrx::kRuleRayQuery>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
+        tr.step<false, false, swrx::kRuleRayQuery, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
       tracing = false;
     // Lanes whose ray is finished wait until shade_batch of them (or every active lane) can shade
     // together: the shading code then runs once for many lanes instead of once per finished ray.
@@ -391,9 +391,10 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_rt_opts* opts, fl
   F.rgba = rgba;
   unsigned long long* cursor = (unsigned long long*)s->d_scratch;
   SWR_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
-  auto kern = k_rt_path<0>;
-  if (opts->blocks_per_sm == 5) kern = k_rt_path<5>;
-  else if (opts->blocks_per_sm == 6) kern = k_rt_path<6>;
+  const bool few = s->dev.num_tris <= swrx::kFewTriangles;
+  auto kern = few ? k_rt_path<0, true> : k_rt_path<0, false>;
+  if (opts->blocks_per_sm == 5) kern = few ? k_rt_path<5, true> : k_rt_path<5, false>;
+  else if (opts->blocks_per_sm == 6) kern = few ? k_rt_path<6, true> : k_rt_path<6, false>;
   int per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0));
   per_sm = std::max(per_sm, 1);

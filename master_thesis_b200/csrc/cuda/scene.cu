@@ -148,7 +148,7 @@ int device_input(const float* p, size_t bytes, cudaStream_t stream, void** tmp, 
 // with one atomic on the cursor, so lanes stay busy while long rays are still walking the tree.
 constexpr unsigned kRefill = 8;
 
-template <bool kStats, int kRule = swrx::kRuleReference>
+template <bool kStats, int kRule, bool kTriLoop>
 __global__ void __launch_bounds__(kTraceBlock, 10)
     k_trace_closest(DevScene sc, const float4* __restrict__ ro, const float4* __restrict__ rd,
                     uint64_t n, uint4* __restrict__ out, uint2* __restrict__ counts,
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kTraceBlock, 10)
       if (exhausted) break;
       continue;
     }
-    if (active && tr.template step<kStats, false, kRule>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
+    if (active && tr.template step<kStats, false, kRule, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
       active = false;
       unwritten = true;
     }
@@ -249,25 +249,19 @@ int trace_impl(swr_scene* s, const float* ray_o, const float* ray_d, uint64_t n,
   }
   unsigned long long* cursor = (unsigned long long*)s->d_scratch;
   SWR_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
-  int per_sm = 0;
-  const bool rq = rule == swrx::kRuleRayQuery;
-  if (rq)
-    SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, k_trace_closest<false, swrx::kRuleRayQuery>, kTraceBlock, 0));
+  const bool few = s->dev.num_tris <= swrx::kFewTrianglesQuery;
+  auto kern = few ? k_trace_closest<false, swrx::kRuleReference, true>
+                  : k_trace_closest<false, swrx::kRuleReference, false>;
+  if (rule == swrx::kRuleRayQuery)
+    kern = few ? k_trace_closest<false, swrx::kRuleRayQuery, true> : k_trace_closest<false, swrx::kRuleRayQuery, false>;
   else if (counts)
-    SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_closest<true>, kTraceBlock, 0));
-  else
-    SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_closest<false>, kTraceBlock, 0));
+    kern = few ? k_trace_closest<true, swrx::kRuleReference, true> : k_trace_closest<true, swrx::kRuleReference, false>;
+  int per_sm = 0;
+  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));
   per_sm = std::max(per_sm, 1);
   const uint64_t max_blocks = (n + kTraceBlock - 1) / kTraceBlock;
   const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)s->num_sms * per_sm, max_blocks);
-  if (rq)
-    k_trace_closest<false, swrx::kRuleRayQuery>
-        <<<grid, kTraceBlock, 0, stream>>>(s->dev, dro, drd, n, dout, nullptr, cursor);
-  else if (counts)
-    k_trace_closest<true><<<grid, kTraceBlock, 0, stream>>>(s->dev, dro, drd, n, dout, dcnt, cursor);
-  else
-    k_trace_closest<false><<<grid, kTraceBlock, 0, stream>>>(s->dev, dro, drd, n, dout, nullptr, cursor);
+  kern<<<grid, kTraceBlock, 0, stream>>>(s->dev, dro, drd, n, dout, dcnt, cursor);
   SWR_CUDA(cudaGetLastError());
   if (hh) SWR_CUDA(cudaMemcpyAsync(out, dout, rb, cudaMemcpyDeviceToHost, stream));
   if (hc) SWR_CUDA(cudaMemcpyAsync(counts, dcnt, (size_t)n * 8, cudaMemcpyDeviceToHost, stream));

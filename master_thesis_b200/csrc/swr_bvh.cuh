@@ -43,6 +43,19 @@ namespace swrx {
 
 constexpr int kNodeF4 = 5;
 constexpr int kTriF4 = 3;
+// Lanes of a warp with a triangle left that keep a step testing (kTriLoop). RayTrace frame and path
+// traced image of the Cornell box, ms: 1.07 and 0.94 without the loop; 0.86 and 0.85 with 2 lanes,
+// 0.88 and 0.84 with 4, 0.91 and 0.85 with 6, 0.96 and 0.85 with 10.
+constexpr int kTriLoopLanes = 4;
+// Scenes of at most this many triangles take the kernels with kTriLoop: their trees are a few levels
+// deep and their rays test more triangles than nodes (Cornell: 3.5 and 1.4). Image, RayTrace frame,
+// bidirectional image, adjoint: Cornell -10, -17, -7, -15 %; 1,000 triangles -2 to -8 %; 2,700 to
+// 47,000 triangles within 2 % either way; 200,000 triangles and terrains +3 % and more.
+constexpr uint32_t kFewTriangles = 2048;
+// The same for closest-hit queries, whose rays are less alike: Cornell -16, 1,000 triangles -10,
+// 5,000 -5, 30,000 and 47,000 -2 %, a 2.4 M-triangle terrain +1.5 %. Batches always take it (64
+// uneven scenes of 1,000 to 50,000 triangles: 1.82 -> 1.78 ms).
+constexpr uint32_t kFewTrianglesQuery = 1u << 16;
 constexpr int kTraceThreads = 128;  // block size of every traversal kernel
 constexpr int kStackShared = 8;   // stack entries per thread kept in shared memory
 // Shared memory of a traversal kernel: rows of one 8-byte entry per thread. Rows 0..7 are the top
@@ -349,12 +362,50 @@ struct Traversal {
     return h;
   }
 
+  template <bool kStats, int kRule>
+  SWR_HD void test_triangle(const float4* __restrict__ tris, const float* __restrict__ tri_boxes,
+                            const float* __restrict__ obj_boxes, uint2* mem, TraceStats* stats) {
+    do {
+      const uint32_t j = (uint32_t)ffs(tg.y) - 1u;
+      tg.y &= tg.y - 1u;
+      const uint32_t s = tg.x + j;
+      if (kStats) stats->tris++;
+      const float4* tp = tris + (size_t)s * kTriF4;
+      const float4 a = ldg4(tp + 0), b = ldg4(tp + 1), c = ldg4(tp + 2);
+      float t, d2;
+      if (!ref_intersect(o, d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), t, d2)) break;
+      const uint2 w = st.get(mem, kRowHit);  // (slot, t) of the best hit so far
+      if (kRule == kRuleRayQuery) {
+        if (!(t >= kRqTmin && t <= kRqTmax)) break;
+        const float bt = bits2f(w.y);
+        if (!(t < bt || (t == bt && f2bits(c.y) < key_of<kRule>(w.x, tris)))) break;
+        st.set(mem, kRowHit, make_uint2(s, f2bits(t)));
+        tprune = t * kPruneSlack;
+        break;
+      }
+      const uint2 v = st.get(mem, kRowDist);
+      const float bd2 = bits2f(v.x);
+      if (!(d2 < bd2 || (d2 == bd2 && f2bits(c.z) < key_of<kRule>(w.x, tris)))) break;
+      if ((v.y & kStrict) && !boxes_hit(s, tris, tri_boxes, obj_boxes)) break;
+      st.set(mem, kRowHit, make_uint2(s, f2bits(t)));
+      st.set(mem, kRowDist, make_uint2(f2bits(d2), v.y));
+      tprune = t * kPruneSlack;
+      if (v.y & kAny) {  // occluded: drop the remaining work so the pop below ends the query
+        ng.y = 0u;
+        tg.y = 0u;
+        st.clear(mem);
+      }
+    } while (false);
+  }
+
   // kPostpone: triangle postponing. While fewer than a fifth of the warp's active lanes have
   // triangles to test, a lane that could still expand nodes parks its triangle group on its
   // stack, so the warp runs one phase at a time. Without it a lane with pending triangles tests
   // one of them per step and a lane without expands a node. (The visit order never changes the
   // result: the closest hit is an arg-min over the same candidates.)
-  template <bool kStats, bool kPostpone = false, int kRule = kRuleReference>
+  // kTriLoop: the lanes with more triangles go on testing them while enough of the warp's lanes
+  // have some (below).
+  template <bool kStats, bool kPostpone = false, int kRule = kRuleReference, bool kTriLoop = false>
   SWR_HD bool step(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                    const float* __restrict__ tri_boxes, const float* __restrict__ obj_boxes,
                    uint2* mem, TraceStats* stats) {
@@ -443,41 +494,22 @@ struct Traversal {
       tri_now = true;
     }
 
-    // At most one triangle per step: a lane with many candidate triangles then holds the warp
-    // for one test per step while the other lanes go on expanding nodes (measured on the
-    // terrain workload: 24.5 ms per image against 28.4 ms when a step tests all of them).
-    do {
-      if (!(tri_now && tg.y)) break;
-      const uint32_t j = (uint32_t)ffs(tg.y) - 1u;
-      tg.y &= tg.y - 1u;
-      const uint32_t s = tg.x + j;
-      if (kStats) stats->tris++;
-      const float4* tp = tris + (size_t)s * kTriF4;
-      const float4 a = ldg4(tp + 0), b = ldg4(tp + 1), c = ldg4(tp + 2);
-      float t, d2;
-      if (!ref_intersect(o, d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), t, d2)) break;
-      const uint2 w = st.get(mem, kRowHit);  // (slot, t) of the best hit so far
-      if (kRule == kRuleRayQuery) {
-        if (!(t >= kRqTmin && t <= kRqTmax)) break;
-        const float bt = bits2f(w.y);
-        if (!(t < bt || (t == bt && f2bits(c.y) < key_of<kRule>(w.x, tris)))) break;
-        st.set(mem, kRowHit, make_uint2(s, f2bits(t)));
-        tprune = t * kPruneSlack;
-        break;
+    // One triangle per step: a lane with many candidate triangles then holds the warp for one test
+    // per step while the other lanes go on expanding nodes (terrain image: testing all of them in the
+    // step cost 16 %). With kTriLoop the step goes on as long as kTriLoopLanes lanes have a triangle
+    // left: where nodes are few and most steps test triangles, the loop around the step (refill and
+    // stage ballots) is what a test costs. See kFewTriangles.
+    if (tri_now && tg.y) {
+      for (;;) {
+        test_triangle<kStats, kRule>(tris, tri_boxes, obj_boxes, mem, stats);
+        if (!kTriLoop) break;
+        const bool more = tg.y != 0;
+#if defined(__CUDA_ARCH__)
+        if (__popc(__ballot_sync(__activemask(), more)) < kTriLoopLanes) break;
+#endif
+        if (!more) break;
       }
-      const uint2 v = st.get(mem, kRowDist);
-      const float bd2 = bits2f(v.x);
-      if (!(d2 < bd2 || (d2 == bd2 && f2bits(c.z) < key_of<kRule>(w.x, tris)))) break;
-      if ((v.y & kStrict) && !boxes_hit(s, tris, tri_boxes, obj_boxes)) break;
-      st.set(mem, kRowHit, make_uint2(s, f2bits(t)));
-      st.set(mem, kRowDist, make_uint2(f2bits(d2), v.y));
-      tprune = t * kPruneSlack;
-      if (v.y & kAny) {  // occluded: drop the remaining work so the pop below ends the query
-        ng.y = 0u;
-        tg.y = 0u;
-        st.clear(mem);
-      }
-    } while (false);
+    }
 
     if (!(ng.y & 0xFF000000u) && tg.y == 0) {
       if (st.empty(mem)) return true;
