@@ -18,6 +18,7 @@
 #include <memory>
 #include <vector>
 
+#include "../swr_wide.cuh"
 #include "shading.cuh"
 #include "swr_internal.cuh"
 
@@ -322,9 +323,8 @@ __global__ void __launch_bounds__(256, 4) k_bshade(BArgs A, BCtrl* __restrict__ 
   }
 }
 
-// bounce traversal over the shared queue, refilling idle lanes (as the single-scene kernel)
-__global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ ctrl, BQueue q, int parity) {
-  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTB];
+// as the single-scene begin_trace
+__device__ __forceinline__ unsigned begin_trace(const BArgs& A, BCtrl* __restrict__ ctrl, int parity) {
   const int qp = parity ^ 1;
   const unsigned n = ctrl->count[qp];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -337,6 +337,28 @@ __global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ 
     ctrl->count[parity] = 0u;
     ctrl->rays += n;
   }
+  return n;
+}
+
+// bounce traversal of a small shared queue, eight lanes per ray (swr_wide.cuh)
+__global__ void __launch_bounds__(kTB) k_btrace_wide(BArgs A, BCtrl* __restrict__ ctrl, BQueue q, int parity) {
+  __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
+  const unsigned n = begin_trace(A, ctrl, parity);
+  for (unsigned i = swrx::wide_first(); i < n; i += swrx::wide_stride()) {
+    const float4 o = q.o[i], d = q.d[i];
+    const DevScene& sc = A.scenes[A.jobs[__float_as_uint(q.c[i].w) >> 16].scene];
+    const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr);
+    if ((lane() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
+  }
+}
+
+// bounce traversal over the shared queue, refilling idle lanes (as the single-scene kernel)
+__global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ ctrl, BQueue q, int parity) {
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTB];
+  const int qp = parity ^ 1;
+  const unsigned n = begin_trace(A, ctrl, parity);
+  if (n == 0u) return;  // an idle round
   const unsigned ln = lane();
   const unsigned lt = (1u << ln) - 1u;
   swrx::Traversal tr;
@@ -700,7 +722,8 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   k_bcamera<<<bcamera_grid(num_sms, pixels), kTB, 0, stream>>>(A, dctrl);
   SWR_CUDA(cudaGetLastError());
   int per_sm = 0;
-  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_btrace, kTB, 0));
+  auto trace_kernel = capw <= swrx::kWideRays ? k_btrace_wide : k_btrace;  // the queue bounds every round
+  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel, kTB, 0));
   const unsigned tgrid = (unsigned)(num_sms * std::max(per_sm, 1));
   int shade_per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shade_per_sm, k_bshade, 256, 0) != cudaSuccess) {
@@ -723,7 +746,7 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
     for (int k = 0; k < 8; ++k) {
       const int p = k & 1;
       k_bshade<<<sgrid, 256, 0, st>>>(A, ctrl, Qh[p], Qh[p ^ 1], p);
-      k_btrace<<<tgrid, kTB, 0, st>>>(A, ctrl, Qh[p ^ 1], p);
+      trace_kernel<<<tgrid, kTB, 0, st>>>(A, ctrl, Qh[p ^ 1], p);
     }
   };
   if (use_graph) {
@@ -741,13 +764,13 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
       BCtrl* ctrl = dctrl + h;
       // the whole round loop as one graph (a WHILE node over eight rounds and k_bcheck), rebuilt
       // whenever an argument baked into it changes
-      std::vector<char> key(sizeof(A) + sizeof(Qh) + 3 * sizeof(void*));
+      std::vector<char> key(sizeof(A) + sizeof(Qh) + 4 * sizeof(void*));
       {
         char* k = key.data();
         std::memset(k, 0, key.size());
         std::memcpy(k, &A, sizeof(A));
         std::memcpy(k + sizeof(A), Qh, sizeof(Qh));
-        const void* extra[3] = {ctrl, (void*)(uintptr_t)sgrid, (void*)(uintptr_t)tgrid};
+        const void* extra[4] = {ctrl, (void*)(uintptr_t)sgrid, (void*)(uintptr_t)tgrid, (void*)trace_kernel};
         std::memcpy(k + sizeof(A) + sizeof(Qh), extra, sizeof(extra));
       }
       if (!b->graph[h] || key != b->graph_key[h]) {

@@ -20,6 +20,7 @@
 #include <mutex>
 #include <vector>
 
+#include "../swr_wide.cuh"
 #include "shading.cuh"
 #include "swr_internal.cuh"
 
@@ -117,6 +118,14 @@ constexpr uint32_t kLitClearedByCamera = 32;
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
+// Pixel k's camera record; its samples start dark.
+__device__ __forceinline__ void put_camera_record(const Frame& F, uint32_t k, float4 rec0, float4 rec1) {
+  F.cam[2 * (size_t)k] = rec0;
+  F.cam[2 * (size_t)k + 1] = rec1;
+  if (F.lit && F.lit_words <= kLitClearedByCamera)
+    for (uint32_t w = 0; w < F.lit_words; ++w) F.lit[(size_t)k * F.lit_words + w] = 0u;
+}
+
 // Camera prefix of every pixel of the chunk (PathTracer::renderPixel's ray and the first bounces
 // of traceSinglePath up to the first front-facing hit, path_tracer.cpp:18-27,42-60): the same for
 // every sample of the pixel, so it is traced once per pixel. Persistent with per-lane refill, as
@@ -184,10 +193,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
         }
       }
       if (done) {
-        F.cam[2 * (size_t)k] = rec0;
-        F.cam[2 * (size_t)k + 1] = rec1;
-        if (F.lit && F.lit_words <= kLitClearedByCamera)
-          for (uint32_t w = 0; w < F.lit_words; ++w) F.lit[(size_t)k * F.lit_words + w] = 0u;
+        put_camera_record(F, k, rec0, rec1);
         active = false;
       }
     }
@@ -197,15 +203,48 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
   if (lane == 0 && traced) atomicAdd(&ctrl->rays, (unsigned long long)traced);
 }
 
-// persistent grid of the camera kernel for a chunk of np pixels
-static unsigned camera_grid(const swr_scene* s, uint32_t np) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_camera, kTraceBlock, 0) != cudaSuccess) {
-    cudaGetLastError();
-    per_sm = 1;
+// The camera prefix of a chunk of few pixels, eight lanes per pixel (swr_wide.cuh).
+__global__ void __launch_bounds__(kTraceBlock) k_camera_wide(DevScene sc, Frame F, Ctrl* __restrict__ ctrl) {
+  __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
+  const unsigned first = (lane_id() & 7u) == 0u;  // the lane that writes for its group
+  unsigned traced = 0;
+  for (uint32_t k = swrx::wide_first(); k < F.npix; k += swrx::wide_stride()) {
+    const uint32_t pix = F.pixel0 + k;
+    const f3 d = swrx::primary_dir(F.vi, F.pi, pix % F.W, pix / F.W, F.W, F.H);
+    f3 o = mk(F.org[0], F.org[1], F.org[2]);
+    float4 rec0 = make_float4(0, 0, 0, 0), rec1 = make_float4(0, 0, 0, __uint_as_float(kDeadSlot));
+    for (uint32_t i = 0; i < F.depth; ++i) {
+      const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
+          sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, o, d, stack, nullptr);
+      traced += first;
+      if (h.slot == kDeadSlot) break;
+      const f3 p = swrx::hit_point(o, d, h.t);
+      if (!(swrx::vdot(swrx::shading_normal(sc.tris, sc.shade, h.slot, p), d) > 0.0f)) {
+        rec0 = make_float4(o.x, o.y, o.z, h.t);
+        rec1 = make_float4(d.x, d.y, d.z, __uint_as_float(h.slot | (i << 27)));
+        break;
+      }
+      o = swrx::vadd(p, swrx::vscale(0.01f, d));  // a back face uses up the slot
+    }
+    if (first) put_camera_record(F, k, rec0, rec1);
   }
-  const uint64_t need = ((uint64_t)np + kTraceBlock - 1) / kTraceBlock;
-  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(need, (uint64_t)s->num_sms * std::max(per_sm, 1)));
+  for (int off = 16; off > 0; off >>= 1) traced += __shfl_down_sync(0xffffffffu, traced, off);
+  if (lane_id() == 0 && traced) atomicAdd(&ctrl->rays, (unsigned long long)traced);
+}
+
+// Launches the camera kernel for the F.npix pixels of a chunk.
+static int launch_camera(const swr_scene* s, const Frame& F, Ctrl* ctrl, cudaStream_t st) {
+  const bool wide = F.npix <= swrx::kWideRays;
+  auto kern = wide ? k_camera_wide : k_camera;
+  int per_sm = 0;
+  SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));
+  const unsigned per_block = wide ? swrx::kWideGroups : kTraceBlock;
+  const uint64_t need = ((uint64_t)F.npix + per_block - 1) / per_block;
+  const unsigned grid =
+      (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(need, (uint64_t)s->num_sms * std::max(per_sm, 1)));
+  kern<<<grid, kTraceBlock, 0, st>>>(s->dev, F, ctrl);
+  SWR_CUDA(cudaGetLastError());
+  return SWR_OK;
 }
 
 // One entry of a shading round: a continuing path (its ray and the hit the traversal found) or an
@@ -363,11 +402,9 @@ static unsigned shade_grid_for(const swr_scene* s, uint32_t cap, int block) {
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(need, (uint64_t)s->num_sms * std::max(per_sm, 1)));
 }
 
-template <bool kStats>
-__global__ void __launch_bounds__(kTraceBlock)
-    k_trace(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
-  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
-  // parity p: trace queue p^1, prepare the injection window of the next shade (parity p^1)
+// Parity p: queue p^1 is traced, and the injection window of the next shade (parity p^1) prepared.
+// Returns the queue's length.
+__device__ __forceinline__ unsigned begin_trace(const Frame& F, Ctrl* __restrict__ ctrl, int parity) {
   const int qp = parity ^ 1;
   const unsigned n = ctrl->count[qp];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -382,6 +419,44 @@ __global__ void __launch_bounds__(kTraceBlock)
     ctrl->bounce_rays += n;
     if (ctrl->first_n == 0u) ctrl->first_n = n;
   }
+  return n;
+}
+
+// Node and triangle counts of a launch.
+__device__ __forceinline__ void add_stats(Ctrl* __restrict__ ctrl, const swrx::TraceStats& st) {
+  unsigned long long nv = st.nodes, tv = st.tris;
+  for (int off = 16; off > 0; off >>= 1) {
+    nv += __shfl_down_sync(0xffffffffu, nv, off);
+    tv += __shfl_down_sync(0xffffffffu, tv, off);
+  }
+  if (lane_id() == 0) {
+    atomicAdd(&ctrl->nodes, nv);
+    atomicAdd(&ctrl->tris, tv);
+  }
+}
+
+// Bounce traversal of a small queue, eight lanes per ray (swr_wide.cuh).
+template <bool kStats>
+__global__ void __launch_bounds__(kTraceBlock)
+    k_trace_wide(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
+  __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
+  const unsigned n = begin_trace(F, ctrl, parity);
+  swrx::TraceStats st{0, 0};
+  for (unsigned i = swrx::wide_first(); i < n; i += swrx::wide_stride()) {
+    const float4 o = q.o[i], d = q.d[i];
+    const swrx::WideHit h = swrx::wide_closest<kStats, swrx::kRuleReference>(
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, &st);
+    if ((lane_id() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
+  }
+  if (kStats) add_stats(ctrl, st);
+}
+
+template <bool kStats>
+__global__ void __launch_bounds__(kTraceBlock)
+    k_trace(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
+  __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
+  const int qp = parity ^ 1;
+  const unsigned n = begin_trace(F, ctrl, parity);
   swrx::Traversal::prepare(stack);
   swrx::TraceStats st{0, 0};
   for (;;) {
@@ -398,17 +473,7 @@ __global__ void __launch_bounds__(kTraceBlock)
       q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
     }
   }
-  if (kStats) {
-    unsigned long long nv = st.nodes, tv = st.tris;
-    for (int off = 16; off > 0; off >>= 1) {
-      nv += __shfl_down_sync(0xffffffffu, nv, off);
-      tv += __shfl_down_sync(0xffffffffu, tv, off);
-    }
-    if (lane_id() == 0) {
-      atomicAdd(&ctrl->nodes, nv);
-      atomicAdd(&ctrl->tris, tv);
-    }
-  }
+  if (kStats) add_stats(ctrl, st);
 }
 
 // Persistent traversal with per-lane refill: each lane keeps its own ray's traversal state;
@@ -421,19 +486,8 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_trace_dyn(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTraceBlock];
   const int qp = parity ^ 1;
-  const unsigned n = ctrl->count[qp];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const unsigned long long rem = ctrl->total - ctrl->injected;
-    const unsigned long long room = (unsigned long long)F.capacity - n;
-    const unsigned long long m = rem < room ? rem : room;
-    ctrl->inj_base[qp] = ctrl->injected;
-    ctrl->inj_n[qp] = (unsigned)m;
-    ctrl->injected += m;
-    ctrl->count[parity] = 0u;
-    ctrl->rays += n;
-    ctrl->bounce_rays += n;
-    if (ctrl->first_n == 0u) ctrl->first_n = n;
-  }
+  const unsigned n = begin_trace(F, ctrl, parity);
+  if (n == 0u) return;  // an idle round
   const unsigned lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   swrx::TraceStats st{0, 0};
@@ -480,17 +534,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       unwritten = true;
     }
   }
-  if (kStats) {
-    unsigned long long nv = st.nodes, tv = st.tris;
-    for (int off = 16; off > 0; off >>= 1) {
-      nv += __shfl_down_sync(0xffffffffu, nv, off);
-      tv += __shfl_down_sync(0xffffffffu, tv, off);
-    }
-    if (lane == 0) {
-      atomicAdd(&ctrl->nodes, nv);
-      atomicAdd(&ctrl->tris, tv);
-    }
-  }
+  if (kStats) add_stats(ctrl, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -992,11 +1036,10 @@ __global__ void __launch_bounds__(256) k_resolve(Frame F, float* __restrict__ im
 }
 
 struct Workspace {
-  size_t qbytes = 0, cam_px = 0, contrib_n = 0, lit_n = 0, stage_n = 0, bd_vtx_n = 0, bd_head_n = 0;
+  size_t qbytes = 0, cam_bytes = 0, contrib_n = 0, stage_n = 0, bd_vtx_n = 0, bd_head_n = 0;
   void* qbuf = nullptr;
-  void* cam = nullptr;
+  void* cam = nullptr;  // camera records, then (wavefront renders) the lit bits
   void* contrib = nullptr;
-  void* lit = nullptr;
   void* stage = nullptr;  // device image for callers that pass a host output buffer
   void* bd_vtx = nullptr;   // bidirectional tracer: per-sample vertex tables
   void* bd_head = nullptr;  // bidirectional tracer: per-sample vertex counts
@@ -1015,13 +1058,13 @@ struct Workspace {
   cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
 };
 
-// End of one iteration of the device-side round loop (eight shade/trace rounds, after which the
-// next shade reads parity 0): continue while paths are queued or samples wait for injection; stop
+// End of one iteration of the device-side round loop (an even number of shade/trace rounds, so that
+// the next shade reads parity 0): continue while paths are queued or samples wait for injection; stop
 // with status 1 once the proven bound on rounds is exceeded (never reached unless the wavefront
 // logic is broken), so the loop always ends.
-__global__ void k_round_check(Ctrl* __restrict__ ctrl, cudaGraphConditionalHandle loop) {
+__global__ void k_round_check(Ctrl* __restrict__ ctrl, cudaGraphConditionalHandle loop, unsigned rounds) {
   Ctrl& c = *ctrl;
-  c.rounds += 8;
+  c.rounds += rounds;
   const bool drained = c.count[0] == 0u && c.inj_n[0] == 0u && c.injected == c.total;
   unsigned go = drained ? 0u : 1u;
   if (!drained && c.rounds > c.max_rounds) {
@@ -1034,10 +1077,10 @@ __global__ void k_round_check(Ctrl* __restrict__ ctrl, cudaGraphConditionalHandl
 constexpr size_t kGraphsKept = 4;
 
 // The round-loop graph for `key` from the cache (built when missing, evicting the least recently
-// used beyond kGraphsKept): a WHILE node whose body is `rounds` (eight shade/trace rounds, enqueued
+// used beyond kGraphsKept): a WHILE node whose body is `rounds` (num_rounds shade/trace rounds, enqueued
 // on the given stream) followed by k_round_check. The key holds every argument baked into it.
 template <class Enqueue>
-int round_loop_graph(Workspace* ws, int slot, const std::vector<char>& key, Ctrl* ctrl, Enqueue rounds,
+int round_loop_graph(Workspace* ws, int slot, const std::vector<char>& key, Ctrl* ctrl, unsigned num_rounds, Enqueue rounds,
                      cudaGraphExec_t* out) {
   auto& cache = ws->graphs[slot];
   for (auto& e : cache)
@@ -1063,7 +1106,7 @@ int round_loop_graph(Workspace* ws, int slot, const std::vector<char>& key, Ctrl
     SWR_CUDA(cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal));
     rounds(cs);
-    k_round_check<<<1, 1, 0, cs>>>(ctrl, loop);
+    k_round_check<<<1, 1, 0, cs>>>(ctrl, loop, num_rounds);
     cudaGraph_t captured = nullptr;
     SWR_CUDA(cudaStreamEndCapture(cs, &captured));
     SWR_CUDA(cudaGraphInstantiate(&exec, g, 0));
@@ -1242,9 +1285,10 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   cap = std::max<uint32_t>(32, (cap + 255u) & ~255u);
   const size_t qbytes = (size_t)cap * kPathBytes * 2;
   if ((rc = ensure(&ws->qbuf, ws->qbytes, qbytes, 1))) return rc;
-  if ((rc = ensure(&ws->cam, ws->cam_px, px_per_chunk, 2 * sizeof(float4)))) return rc;
+  const size_t cam_bytes = px_per_chunk * 2 * sizeof(float4);
+  const size_t lit_bytes = px_per_chunk * lit_words_of(o->spp) * sizeof(uint32_t);
+  if ((rc = ensure(&ws->cam, ws->cam_bytes, cam_bytes + lit_bytes, 1))) return rc;
   if ((rc = ensure(&ws->contrib, ws->contrib_n, px_per_chunk * o->spp, sizeof(float4)))) return rc;
-  if ((rc = ensure(&ws->lit, ws->lit_n, px_per_chunk * lit_words_of(o->spp), sizeof(uint32_t)))) return rc;
   if (!ws->ctrl) {
     SWR_CUDA(cudaMalloc(&ws->ctrl, 4 * sizeof(Ctrl)));
     SWR_CUDA(cudaMallocHost(&ws->host_ctrl, 4 * sizeof(Ctrl)));
@@ -1292,7 +1336,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   F.capacity = cap;
   F.cam = (float4*)ws->cam;
   F.contrib = (float4*)ws->contrib;
-  F.lit = (uint32_t*)ws->lit;
+  F.lit = (uint32_t*)((char*)ws->cam + cam_bytes);
   F.lit_words = lit_words_of(o->spp);
   set_div_spp(F, px_per_chunk);
 
@@ -1314,6 +1358,8 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       break;
     default: return set_error(SWR_ERR_INVALID, "swr: trace_blocks must be 0, 9 or 10");
   }
+  if (cap <= swrx::kWideRays && !postpone && o->trace_blocks == 0)  // bounds every round
+    trace_kernel = count ? k_trace_wide<true> : k_trace_wide<false>;
   if (static_fetch) trace_kernel = count ? k_trace<true> : k_trace<false>;
   if (o->refill > 32) return set_error(SWR_ERR_INVALID, "swr: refill must be 0..32");
   F.refill = o->refill ? o->refill : 8;
@@ -1358,7 +1404,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     SWR_CUDA(cudaMemcpyAsync(ctrl, ws->host_ctrl + h, sizeof(Ctrl), cudaMemcpyHostToDevice, st));
     P.h2d_bytes += sizeof(Ctrl);
     if ((rc = clear_samples(s, Fh, want_samples, st))) return rc;
-    k_camera<<<camera_grid(s, n), kTraceBlock, 0, st>>>(s->dev, Fh, ctrl);
+    if ((rc = launch_camera(s, Fh, ctrl, st))) return rc;
     SWR_CUDA(cudaGetLastError());
     // the shading and traversal kernels read the first pixel from the control block, so their
     // arguments (and a graph made of them) are the same for every chunk
@@ -1366,21 +1412,24 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     FR.pixel0 = 0;
     FR.npix = 0;
     const unsigned sgrid = shade_grid_for(s, capw, block);
-    std::vector<char> key(sizeof(DevScene) + sizeof(Frame) + sizeof(Qh) + 5 * sizeof(void*));
+    // rounds per iteration of the loop: what drains a chunk that is injected at once (its paths end
+    // within max_depth rounds), when that is fewer than eight: an idle round takes about 5 us
+    const unsigned body = (total <= capw && o->max_depth <= 8) ? (o->max_depth + 1u) & ~1u : 8u;
+    std::vector<char> key(sizeof(DevScene) + sizeof(Frame) + sizeof(Qh) + 6 * sizeof(void*));
     {
       char* kp = key.data();
       std::memset(kp, 0, key.size());
       std::memcpy(kp, &s->dev, sizeof(DevScene));
       std::memcpy(kp + sizeof(DevScene), &FR, sizeof(Frame));
       std::memcpy(kp + sizeof(DevScene) + sizeof(Frame), Qh, sizeof(Qh));
-      const void* extra[5] = {ctrl, (void*)trace_kernel, (void*)(uintptr_t)block, (void*)(uintptr_t)trace_grid,
-                              (void*)(uintptr_t)sgrid};
+      const void* extra[6] = {ctrl, (void*)trace_kernel, (void*)(uintptr_t)block, (void*)(uintptr_t)trace_grid,
+                              (void*)(uintptr_t)sgrid, (void*)(uintptr_t)body};
       std::memcpy(kp + sizeof(DevScene) + sizeof(Frame) + sizeof(Qh), extra, sizeof(extra));
     }
     cudaGraphExec_t graph = nullptr;
-    int grc = round_loop_graph(ws, h, key, ctrl, [&](cudaStream_t cs) {
-      for (int c = 0; c < 8; ++c) {
-        const int q = c & 1;
+    int grc = round_loop_graph(ws, h, key, ctrl, body, [&](cudaStream_t cs) {
+      for (unsigned c = 0; c < body; ++c) {
+        const int q = (int)(c & 1u);
         switch (block) {
           case 128: k_shade<128><<<sgrid, 128, 0, cs>>>(s->dev, FR, ctrl, Qh[q], Qh[q ^ 1], q); break;
           case 512: k_shade<512><<<sgrid, 512, 0, cs>>>(s->dev, FR, ctrl, Qh[q], Qh[q ^ 1], q); break;
@@ -1413,7 +1462,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     P.node_visits += hc.nodes;
     P.tri_tests += hc.tris;
     P.iterations += hc.rounds;
-    P.launches += 2 + 2 * hc.rounds + hc.rounds / 8;  // camera, resolve, rounds, checks
+    P.launches += 2 + 2 * hc.rounds + hc.rounds / 8;  // camera, resolve, rounds, checks (at least)
     P.trace_launches += hc.rounds;
     return SWR_OK;
   };
@@ -1475,7 +1524,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       P.h2d_bytes += sizeof(Ctrl);
       if ((rc = clear_samples(s, F, want_samples, stream))) return rc;
       SWR_CUDA(timer.begin(stream, kTimeCamera));
-      k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl);
+      if ((rc = launch_camera(s, F, ws->ctrl, stream))) return rc;
       SWR_CUDA(timer.end(stream));
       SWR_CUDA(cudaGetLastError());
       P.launches++;
@@ -1556,7 +1605,6 @@ void free_workspace(swr_scene* s) {
   if (ws->qbuf) cudaFree(ws->qbuf);
   if (ws->cam) cudaFree(ws->cam);
   if (ws->contrib) cudaFree(ws->contrib);
-  if (ws->lit) cudaFree(ws->lit);
   if (ws->stage) cudaFree(ws->stage);
   if (ws->bd_vtx) cudaFree(ws->bd_vtx);
   if (ws->bd_head) cudaFree(ws->bd_head);
@@ -1597,7 +1645,7 @@ int render_adjoint_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
   RenderWorkspace* ws = workspace_of(s);
   const uint64_t npix_total = (uint64_t)o->width * o->height;
   const uint64_t px_per_chunk = std::max<uint64_t>(1, std::min<uint64_t>(npix_total, kChunkSamples / o->spp));
-  if ((rc = ensure(&ws->cam, ws->cam_px, px_per_chunk, 2 * sizeof(float4)))) return rc;
+  if ((rc = ensure(&ws->cam, ws->cam_bytes, px_per_chunk * 2 * sizeof(float4), 1))) return rc;
   if (!ws->ctrl) {
     SWR_CUDA(cudaMalloc(&ws->ctrl, 4 * sizeof(Ctrl)));
     SWR_CUDA(cudaMallocHost(&ws->host_ctrl, 4 * sizeof(Ctrl)));
@@ -1644,7 +1692,7 @@ int render_adjoint_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
     SWR_CUDA(cudaStreamSynchronize(stream));  // the pinned control block may still be in flight
     *ws->host_ctrl = init;
     SWR_CUDA(cudaMemcpyAsync(ws->ctrl, ws->host_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, stream));
-    k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl);
+    if ((rc = launch_camera(s, F, ws->ctrl, stream))) return rc;
     kern<<<grid, kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl, dl, g_alb, g_em);
     SWR_CUDA(cudaGetLastError());
   }
@@ -1700,7 +1748,7 @@ int render_bdpt_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts*
                                       : std::max<uint64_t>(1u << 14, kBdptTableBytes / (48 * slots));
   const uint64_t px_per_chunk = std::max<uint64_t>(1, std::min<uint64_t>(npix_total, chunk / o->spp));
   int rc;
-  if ((rc = ensure(&ws->cam, ws->cam_px, px_per_chunk, 2 * sizeof(float4)))) return rc;
+  if ((rc = ensure(&ws->cam, ws->cam_bytes, px_per_chunk * 2 * sizeof(float4), 1))) return rc;
   if ((rc = ensure(&ws->contrib, ws->contrib_n, px_per_chunk * o->spp, sizeof(float4)))) return rc;
   if ((rc = ensure(&ws->bd_vtx, ws->bd_vtx_n, px_per_chunk * o->spp * 3 * slots, sizeof(float4)))) return rc;
   if ((rc = ensure(&ws->bd_head, ws->bd_head_n, px_per_chunk * o->spp, sizeof(uint4)))) return rc;
@@ -1763,7 +1811,7 @@ int render_bdpt_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts*
     SWR_CUDA(cudaStreamSynchronize(stream));  // the pinned control block may still be in flight
     *ws->host_ctrl = init;
     SWR_CUDA(cudaMemcpyAsync(ws->ctrl, ws->host_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, stream));
-    k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl);
+    if ((rc = launch_camera(s, F, ws->ctrl, stream))) return rc;
     B.nsamp = np * o->spp;
     kern<<<grid, kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl, B);
     kconn<<<grid_c, kTraceBlock, 0, stream>>>(s->dev, F, ws->ctrl, B);
@@ -1924,7 +1972,7 @@ int render_noalloc_impl(swr_scene* s, const swr_camera* cam, const swr_render_op
     // pageable source: the copy has been taken when the call returns
     SWR_CUDA(cudaMemcpyAsync(ctrl, &init, sizeof(Ctrl), cudaMemcpyHostToDevice, stream));
     if ((rc = clear_samples(s, F, want_samples, stream))) return rc;
-    k_camera<<<camera_grid(s, np), kTraceBlock, 0, stream>>>(s->dev, F, ctrl);
+    if ((rc = launch_camera(s, F, ctrl, stream))) return rc;
     SWR_CUDA(cudaGetLastError());
     uint64_t k = 0;
     const uint64_t max_rounds = (total / cap + 2) * (uint64_t)(o->max_depth + 2) + 64;

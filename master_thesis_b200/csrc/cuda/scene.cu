@@ -7,6 +7,7 @@
 
 #include "../host/capi_common.h"
 #include "../host/scene_pack.h"
+#include "../swr_wide.cuh"
 #include "build_device.h"
 #include "swr_internal.cuh"
 
@@ -207,6 +208,33 @@ __global__ void __launch_bounds__(kTraceBlock, 10)
   }
 }
 
+// The same for few rays, eight lanes each (swr_wide.cuh).
+template <bool kStats, int kRule>
+__global__ void __launch_bounds__(kTraceBlock)
+    k_trace_closest_wide(DevScene sc, const float4* __restrict__ ro, const float4* __restrict__ rd, uint64_t n,
+                         uint4* __restrict__ out, uint2* __restrict__ counts, unsigned long long*) {
+  __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
+  for (uint32_t i = swrx::wide_first(); i < n; i += swrx::wide_stride()) {
+    const float4 o = ro[i], d = rd[i];
+    swrx::TraceStats st{0, 0};
+    const swrx::WideHit h =
+        swrx::wide_closest<kStats, kRule>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, swrx::mk(o.x, o.y, o.z),
+                                          swrx::mk(d.x, d.y, d.z), stack, &st);
+    if (kStats) st.tris = __reduce_add_sync(0xFFu << (threadIdx.x & 24u), st.tris);
+    if ((threadIdx.x & 7u) == 0u) {
+      uint4 r = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, __float_as_uint(h.d2), __float_as_uint(h.t));
+      if (h.slot != 0xFFFFFFFFu) {
+        const float4 c = __ldg(sc.tris + 3 * (size_t)h.slot + 2);
+        r.x = __float_as_uint(c.y);
+        r.y = __float_as_uint(c.w);
+      }
+      if (kRule == swrx::kRuleRayQuery) r.z = __float_as_uint(INFINITY);
+      out[i] = r;
+      if (kStats) counts[i] = make_uint2(st.nodes, st.tris);
+    }
+  }
+}
+
 int trace_impl(swr_scene* s, const float* ray_o, const float* ray_d, uint64_t n, swr_hit* out,
                uint32_t* counts, void* stream_, int rule = swrx::kRuleReference) {
   if (!s || !ray_o || !ray_d || !out) return set_error(SWR_ERR_INVALID, "swr: null argument");
@@ -248,7 +276,8 @@ int trace_impl(swr_scene* s, const float* ray_o, const float* ray_d, uint64_t n,
     return set_error(SWR_ERR_INVALID, "swr: ray and hit buffers must be 16-byte aligned");
   }
   unsigned long long* cursor = (unsigned long long*)s->d_scratch;
-  SWR_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
+  const bool wide = n <= swrx::kWideRays;
+  if (!wide) SWR_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
   const bool few = s->dev.num_tris <= swrx::kFewTrianglesQuery;
   auto kern = few ? k_trace_closest<false, swrx::kRuleReference, true>
                   : k_trace_closest<false, swrx::kRuleReference, false>;
@@ -256,10 +285,16 @@ int trace_impl(swr_scene* s, const float* ray_o, const float* ray_d, uint64_t n,
     kern = few ? k_trace_closest<false, swrx::kRuleRayQuery, true> : k_trace_closest<false, swrx::kRuleRayQuery, false>;
   else if (counts)
     kern = few ? k_trace_closest<true, swrx::kRuleReference, true> : k_trace_closest<true, swrx::kRuleReference, false>;
+  if (wide) {
+    kern = k_trace_closest_wide<false, swrx::kRuleReference>;
+    if (rule == swrx::kRuleRayQuery) kern = k_trace_closest_wide<false, swrx::kRuleRayQuery>;
+    else if (counts) kern = k_trace_closest_wide<true, swrx::kRuleReference>;
+  }
   int per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));
   per_sm = std::max(per_sm, 1);
-  const uint64_t max_blocks = (n + kTraceBlock - 1) / kTraceBlock;
+  const unsigned per_block = wide ? swrx::kWideGroups : kTraceBlock;
+  const uint64_t max_blocks = (n + per_block - 1) / per_block;
   const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)s->num_sms * per_sm, max_blocks);
   kern<<<grid, kTraceBlock, 0, stream>>>(s->dev, dro, drd, n, dout, dcnt, cursor);
   SWR_CUDA(cudaGetLastError());
