@@ -328,6 +328,16 @@ int swr_render_batch(swr_batch* batch, const swr_batch_job* jobs, uint32_t num_j
 int swr_scene_set_albedo(swr_scene* scene, const float* albedo, void* stream);
 int swr_scene_set_emission(swr_scene* scene, const float* emission, void* stream);
 
+/* swr_scene_set_albedo and swr_scene_set_emission of many scenes in one launch (inverse rendering
+ * sets every scene of a batch before each pass). The scenes differ from each other and are on the
+ * batch's device. */
+typedef struct swr_parameter_job {
+  swr_scene* scene;
+  const float* albedo;
+  const float* emission;
+} swr_parameter_job;
+int swr_batch_set_parameters(swr_batch* batch, const swr_parameter_job* jobs, uint32_t num_jobs, void* stream);
+
 /* Gradient of sum_p dl_dimage[p] . image[p] for the SWR_MODE_PHYSICAL image that swr_render
  * produces with the same scene, camera and opts (same seed = the same sampled paths), with respect
  * to the per-triangle albedo ([num_triangles*3] by triangle id) and the per-object emission

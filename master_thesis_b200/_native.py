@@ -117,6 +117,10 @@ class AdjointJob(ctypes.Structure):
                 ("dl_dalbedo", ctypes.c_void_p), ("dl_demission", ctypes.c_void_p)]
 
 
+class ParameterJob(ctypes.Structure):
+    _fields_ = [("scene", ctypes.c_void_p), ("albedo", ctypes.c_void_p), ("emission", ctypes.c_void_p)]
+
+
 BATCH_NO_GRAPH = 1
 
 
@@ -178,6 +182,7 @@ SIGNATURES = {
     "swr_render_adjoint_batch": (I, [P, ctypes.POINTER(AdjointJob), U32, ctypes.POINTER(BatchOpts), P]),
     "swr_scene_set_albedo": (I, [P, P, P]),
     "swr_scene_set_emission": (I, [P, P, P]),
+    "swr_batch_set_parameters": (I, [P, ctypes.POINTER(ParameterJob), U32, P]),
     "swr_render_adjoint": (I, [P, ctypes.POINTER(Camera), ctypes.POINTER(RenderOpts), P, P, P, P]),
     "swr_render_adjoint_timed": (I, [P, ctypes.POINTER(Camera), ctypes.POINTER(RenderOpts), P, P, P, P,
                                      ctypes.POINTER(ctypes.c_double)]),

@@ -357,6 +357,13 @@ class Batch:
         check(N.lib.swr_render_batch(self._h, arr, len(jobs), ctypes.byref(o), _stream_handle(stream)))
         return outs
 
+    def set_parameters(self, scenes, albedos, emissions, stream=None):
+        """Scene.set_albedo and Scene.set_emission of many scenes (each once) in one launch."""
+        arr = (N.ParameterJob * len(scenes))()
+        for k, sc in enumerate(scenes):
+            arr[k].scene, arr[k].albedo, arr[k].emission = sc.handle, ptr(albedos[k]), ptr(emissions[k])
+        check(N.lib.swr_batch_set_parameters(self._h, arr, len(scenes), _stream_handle(stream)))
+
     def render_adjoint(self, jobs, refill=0, stream=None, shade_batch=0):
         """Path-replay adjoint of many physical-mode jobs in one launch. jobs: dicts as for render
         plus dl_dimage (cuda tensor [h, w, 3]) and optionally grad_albedo / grad_emission (cuda

@@ -544,6 +544,55 @@ __global__ void k_bresolve(BArgs A) {
     o[k] = __double2float_rn((double)(long long)acc[k] / kFix * s);
 }
 
+// One scene's parameters for k_set_parameters: its blocks cover its triangles, then its objects.
+struct ParamJob {
+  const uint32_t* slot_of;
+  const float *albedo, *emission;  // by triangle id, by object
+  float* by_slot;
+  float4* mats;
+  uint32_t num_tris, num_objects, block0;
+};
+constexpr uint32_t kParamBlock = 256;
+
+// Latency- and launch-bound: 16 scenes took 32 launches of 2 us, 64 per inverse-rendering step, with
+// a host call each; one launch takes 4 us.
+__global__ void __launch_bounds__(kParamBlock) k_set_parameters(const ParamJob* __restrict__ jobs, uint32_t n) {
+  uint32_t lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (jobs[mid].block0 <= blockIdx.x) lo = mid;
+    else hi = mid;
+  }
+  const ParamJob J = jobs[lo];
+  const uint32_t tri_blocks = (J.num_tris + kParamBlock - 1) / kParamBlock;
+  const uint32_t b = blockIdx.x - J.block0;
+  if (b < tri_blocks) {
+    const uint32_t t = b * kParamBlock + threadIdx.x;
+    if (t >= J.num_tris) return;
+    const uint32_t s = J.slot_of[t];
+    for (int k = 0; k < 3; ++k) J.by_slot[3 * (size_t)s + k] = J.albedo[3 * (size_t)t + k];
+  } else {
+    const uint32_t o = (b - tri_blocks) * kParamBlock + threadIdx.x;
+    if (o >= J.num_objects) return;
+    float4 m = J.mats[3 * (size_t)o + 2];
+    m.x = J.emission[3 * (size_t)o + 0];
+    m.y = J.emission[3 * (size_t)o + 1];
+    m.z = J.emission[3 * (size_t)o + 2];
+    J.mats[3 * (size_t)o + 2] = m;
+  }
+}
+
+// Zeroes many buffers of floats in one launch; blockIdx.y is the buffer.
+struct ZeroJob {
+  float* p;
+  uint64_t n;
+};
+__global__ void k_zero(const ZeroJob* __restrict__ jobs) {
+  const ZeroJob J = jobs[blockIdx.y];
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < J.n; k += (uint64_t)gridDim.x * blockDim.x)
+    J.p[k] = 0.0f;
+}
+
 int ensure_bytes(void** p, size_t& have, size_t want) {
   if (have >= want && *p) return SWR_OK;
   if (*p) cudaFree(*p);
@@ -562,8 +611,9 @@ int ensure_bytes(void** p, size_t& have, size_t want) {
 }  // namespace swr
 
 struct swr_batch {
-  void *qbuf = nullptr, *cam = nullptr, *accum = nullptr, *jobs = nullptr, *scenes = nullptr, *ctrl = nullptr;
-  size_t qbytes = 0, cambytes = 0, accbytes = 0, jobbytes = 0, scenebytes = 0, ctrlbytes = 0;
+  void *qbuf = nullptr, *cam = nullptr, *accum = nullptr, *jobs = nullptr, *scenes = nullptr, *ctrl = nullptr,
+       *params = nullptr;
+  size_t qbytes = 0, cambytes = 0, accbytes = 0, jobbytes = 0, scenebytes = 0, ctrlbytes = 0, parambytes = 0;
   swr::BCtrl* host_ctrl = nullptr;                                  // [4] pinned control blocks
   cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};  // round loop per sub-wavefront
   std::vector<char> graph_key[4];
@@ -641,7 +691,7 @@ void swr_batch_destroy(swr_batch* b) {
     if (b->join[h]) cudaEventDestroy(b->join[h]);
   }
   if (b->fork) cudaEventDestroy(b->fork);
-  for (void* p : {b->qbuf, b->cam, b->accum, b->jobs, b->scenes, b->ctrl})
+  for (void* p : {b->qbuf, b->cam, b->accum, b->jobs, b->scenes, b->ctrl, b->params})
     if (p) cudaFree(p);
   if (b->host_ctrl) cudaFreeHost(b->host_ctrl);
   delete b;
@@ -845,6 +895,46 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   return SWR_OK;
 }
 
+int swr_batch_set_parameters(swr_batch* b, const swr_parameter_job* jobs, uint32_t n, void* stream_) {
+  using namespace swr;
+  if (!b || !jobs || n == 0) return set_error(SWR_ERR_INVALID, "swr: empty batch");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SWR_CUDA(cudaSetDevice(b->device));
+  bool staged = false;  // host buffers take the per-scene calls, which stage them
+  for (uint32_t k = 0; k < n; ++k) {
+    if (!jobs[k].scene || !jobs[k].albedo || !jobs[k].emission) return set_error(SWR_ERR_INVALID, "swr: null argument");
+    if (jobs[k].scene->device != b->device) return set_error(SWR_ERR_INVALID, "swr: batch jobs on another device");
+    staged = staged || is_host_pointer(jobs[k].albedo) || is_host_pointer(jobs[k].emission);
+  }
+  int rc;
+  if (staged) {
+    for (uint32_t k = 0; k < n; ++k) {
+      if ((rc = swr_scene_set_albedo(jobs[k].scene, jobs[k].albedo, stream_))) return rc;
+      if ((rc = swr_scene_set_emission(jobs[k].scene, jobs[k].emission, stream_))) return rc;
+    }
+    return SWR_OK;
+  }
+  try {
+    std::vector<ParamJob> hp(n);
+    uint64_t blocks = 0;
+    for (uint32_t k = 0; k < n; ++k) {
+      swr_scene* s = jobs[k].scene;
+      const uint32_t nt = s->dev.num_tris, no = s->dev.num_objects;
+      hp[k] = {s->dev.slot_of, jobs[k].albedo, jobs[k].emission, (float*)s->d_albedo, (float4*)s->d_mats, nt, no,
+               (uint32_t)blocks};
+      blocks += (nt + kParamBlock - 1) / kParamBlock + (no + kParamBlock - 1) / kParamBlock;
+    }
+    if (blocks > 0x7FFFFFFFull) return set_error(SWR_ERR_UNSUPPORTED, "swr: too many triangles in one call");
+    if ((rc = ensure_bytes(&b->params, b->parambytes, n * sizeof(ParamJob)))) return rc;
+    SWR_CUDA(cudaMemcpyAsync(b->params, hp.data(), n * sizeof(ParamJob), cudaMemcpyHostToDevice, stream));
+    k_set_parameters<<<(unsigned)blocks, kParamBlock, 0, stream>>>((const ParamJob*)b->params, n);
+    SWR_CUDA(cudaGetLastError());
+  } catch (const std::bad_alloc&) {
+    return set_error(SWR_ERR_ALLOC, "swr: host allocation failed");
+  }
+  return SWR_OK;
+}
+
 int swr_render_adjoint_batch(swr_batch* b, const swr_adjoint_job* jobs, uint32_t n, const swr_batch_opts* bo,
                              void* stream_) {
   using namespace swr;
@@ -898,7 +988,17 @@ int swr_render_adjoint_batch(swr_batch* b, const swr_adjoint_job* jobs, uint32_t
   if ((rc = ensure_bytes(&b->ctrl, b->ctrlbytes, 4 * sizeof(BCtrl)))) return rc;
   SWR_CUDA(cudaMemcpyAsync(b->jobs, hj.data(), n * sizeof(BJob), cudaMemcpyHostToDevice, stream));
   SWR_CUDA(cudaMemcpyAsync(b->scenes, hs.data(), hs.size() * sizeof(DevScene), cudaMemcpyHostToDevice, stream));
-  for (auto& z : zero) SWR_CUDA(cudaMemsetAsync(z.first, 0, z.second, stream));
+  // at most 65535 buffers (the grid's second dimension) per launch
+  std::vector<ZeroJob> hz;
+  for (auto& z : zero) hz.push_back({z.first, z.second / sizeof(float)});
+  if ((rc = ensure_bytes(&b->params, b->parambytes, hz.size() * sizeof(ZeroJob)))) return rc;
+  SWR_CUDA(cudaMemcpyAsync(b->params, hz.data(), hz.size() * sizeof(ZeroJob), cudaMemcpyHostToDevice, stream));
+  for (size_t z0 = 0; z0 < hz.size(); z0 += 65535) {
+    const unsigned nz = (unsigned)std::min<size_t>(65535, hz.size() - z0);
+    const unsigned per = std::max(1u, (unsigned)(num_sms * 8) / nz);
+    k_zero<<<dim3(per, nz), 256, 0, stream>>>((const ZeroJob*)b->params + z0);
+    SWR_CUDA(cudaGetLastError());
+  }
   BArgs A;
   std::memset(&A, 0, sizeof(A));
   A.jobs = (const BJob*)b->jobs;

@@ -52,9 +52,7 @@ class _PhysicalRenderBatch(torch.autograd.Function):
     @staticmethod
     def forward(ctx, batch, jobs, adjoint_seeds, *params):
         params = [p.detach().contiguous() for p in params]
-        for k, j in enumerate(jobs):
-            j["scene"].set_albedo(params[2 * k])
-            j["scene"].set_emission(params[2 * k + 1])
+        batch.set_parameters([j["scene"] for j in jobs], params[0::2], params[1::2])
         imgs = batch.render([dict(j, mode=N.MODE_PHYSICAL) for j in jobs])
         ctx.save_for_backward(*params)
         ctx.batch, ctx.jobs, ctx.adjoint_seeds = batch, jobs, adjoint_seeds
@@ -64,9 +62,8 @@ class _PhysicalRenderBatch(torch.autograd.Function):
     def backward(ctx, *grads):
         params = ctx.saved_tensors
         adj = []
+        ctx.batch.set_parameters([j["scene"] for j in ctx.jobs], params[0::2], params[1::2])
         for k, j in enumerate(ctx.jobs):
-            j["scene"].set_albedo(params[2 * k])
-            j["scene"].set_emission(params[2 * k + 1])
             g = grads[k]
             if g is None:
                 g = torch.zeros((j["height"], j["width"], 3), dtype=torch.float32, device=params[2 * k].device)

@@ -1,0 +1,36 @@
+"""One launch that sets the parameters of many scenes against the per-scene calls: triangle and object
+counts around the launch's block size, device and host buffers."""
+import numpy as np
+import pytest
+
+import master_thesis_b200 as swr
+from master_thesis_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("where", ["device", "host"])
+def test_batch_parameters_as_per_scene(where):
+    import torch
+    datas = [scenes.random_scene(40 + k, n)[0] for k, n in enumerate((4, 252, 256, 260, 3000))]
+    rng = np.random.default_rng(2)
+    alb = [rng.uniform(0.05, 0.95, (d.num_triangles, 3)).astype(np.float32) for d in datas]
+    em = [rng.uniform(0.5, 9.0, (d.num_objects, 3)).astype(np.float32) for d in datas]
+    W, H = 24, 16
+    cam = swr.make_camera((4.0, 2.5, 4.0), (-0.75, -0.3), W, H, fov_deg=60.0)
+    one = [swr.Scene(d) for d in datas]
+    many = [swr.Scene(d) for d in datas]
+    give = (lambda a: torch.from_numpy(a).cuda()) if where == "device" else (lambda a: a)
+    for s, a, e in zip(one, alb, em):
+        s.set_albedo(give(a))
+        s.set_emission(give(e))
+    batch = swr.Batch()
+    batch.set_parameters(many, [give(a) for a in alb], [give(e) for e in em])
+    lit = 0
+    for a, b in zip(one, many):
+        x = a.render(cam, W, H, 64, 4, seed=1, mode=swr.MODE_PHYSICAL)
+        assert torch.equal(x, b.render(cam, W, H, 64, 4, seed=1, mode=swr.MODE_PHYSICAL))
+        lit += int(torch.count_nonzero(x))
+    assert lit > 0
+    with pytest.raises(swr.SwrError if hasattr(swr, "SwrError") else Exception):
+        batch.set_parameters([], [], [])
