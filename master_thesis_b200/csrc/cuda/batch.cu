@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ 
       if (exhausted) break;
       continue;
     }
-    if (active && tr.step<false, false, swrx::kRuleReference, true>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
+    if (active && tr.step<false, false, swrx::kRuleReference, true, true>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
       active = false;
       unwritten = true;
     }
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false, swrx::kRuleReference, true>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
+    if (active && tracing && tr.step<false, false, swrx::kRuleReference, true, true>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
       tracing = false;
       if (tr.hit_slot(stack) == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
         active = false;

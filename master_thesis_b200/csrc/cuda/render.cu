@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tr.template step<kStats, kPostpone, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
+    if (active && tr.template step<kStats, kPostpone, swrx::kRuleReference, kTriLoop, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, &st)) {
       active = false;
       unwritten = true;
     }
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
+    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
       tracing = false;
       hslot = tr.hit_slot(stack);
       ht = tr.hit_t(stack);
@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (exhausted) break;
       continue;
     }
-    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
+    if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
       tracing = false;
     const unsigned waiting = __ballot_sync(0xffffffffu, active && !tracing);
     const unsigned inflight = __ballot_sync(0xffffffffu, active && tracing);

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       continue;
     }
     if (active && tracing &&
-        tr.step<false, false, swrx::kRuleRayQuery, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
+        tr.step<false, false, swrx::kRuleRayQuery, kTriLoop, true>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr))
       tracing = false;
     // Lanes whose ray is finished wait until shade_batch of them (or every active lane) can shade
     // together: the shading code then runs once for many lanes instead of once per finished ray.

@@ -362,7 +362,7 @@ struct Traversal {
     return h;
   }
 
-  template <bool kStats, int kRule>
+  template <bool kStats, int kRule, bool kFlat>
   SWR_HD void test_triangle(const float4* __restrict__ tris, const float* __restrict__ tri_boxes,
                             const float* __restrict__ obj_boxes, uint2* mem, TraceStats* stats) {
     do {
@@ -373,7 +373,7 @@ struct Traversal {
       const float4* tp = tris + (size_t)s * kTriF4;
       const float4 a = ldg4(tp + 0), b = ldg4(tp + 1), c = ldg4(tp + 2);
       float t, d2;
-      if (!ref_intersect(o, d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), t, d2)) break;
+      if (!ref_intersect<kFlat>(o, d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), t, d2)) break;
       const uint2 w = st.get(mem, kRowHit);  // (slot, t) of the best hit so far
       if (kRule == kRuleRayQuery) {
         if (!(t >= kRqTmin && t <= kRqTmax)) break;
@@ -405,7 +405,8 @@ struct Traversal {
   // result: the closest hit is an arg-min over the same candidates.)
   // kTriLoop: the lanes with more triangles go on testing them while enough of the warp's lanes
   // have some (below).
-  template <bool kStats, bool kPostpone = false, int kRule = kRuleReference, bool kTriLoop = false>
+  template <bool kStats, bool kPostpone = false, int kRule = kRuleReference, bool kTriLoop = false,
+            bool kFlat = false>
   SWR_HD bool step(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                    const float* __restrict__ tri_boxes, const float* __restrict__ obj_boxes,
                    uint2* mem, TraceStats* stats) {
@@ -501,7 +502,7 @@ struct Traversal {
     // stage ballots) is what a test costs. See kFewTriangles.
     if (tri_now && tg.y) {
       for (;;) {
-        test_triangle<kStats, kRule>(tris, tri_boxes, obj_boxes, mem, stats);
+        test_triangle<kStats, kRule, kFlat>(tris, tri_boxes, obj_boxes, mem, stats);
         if (!kTriLoop) break;
         const bool more = tg.y != 0;
 #if defined(__CUDA_ARCH__)
