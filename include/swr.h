@@ -442,8 +442,8 @@ typedef struct swr_rt_opts {
   uint32_t refill;         /* idle lanes of a warp that take new pixels (1..32), 0 = 4 */
   uint32_t shade_batch;    /* lanes of a warp with a finished ray that shade together (1..32; fewer
                               when no ray of the warp is in flight), 0 = 12 */
-  uint32_t blocks_per_sm;  /* resident blocks per SM targeted by the register budget: 0 (compiler's
-                              choice), 5 or 6 */
+  uint32_t blocks_per_sm;  /* resident blocks per SM targeted by the register budget: 0 (the
+                              library's choice by image and scene size: 5, 6 or 7), 5 or 6 */
   uint32_t reserved;
 } swr_rt_opts;
 

@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ 
 // global samples (refilling idle lanes), find their job by binary search, start from the job's
 // per-pixel camera record and replay the path with the job's scene, seed and Russian roulette,
 // then sweep it into the job's gradient buffers. ctrl->injected is the sample cursor.
-__global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ ctrl) {
+__global__ void __launch_bounds__(kTB, 9) k_badjoint(BArgs A, BCtrl* __restrict__ ctrl) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kTB];
   const unsigned ln = lane();
   const unsigned lt = (1u << ln) - 1u;
@@ -426,8 +426,6 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
   tape.reset();
   const BJob* J = nullptr;
   const DevScene* sc = nullptr;
-  uint32_t pixel = 0, sample = 0, pend_slot = 0;
-  float pend_t = 0.0f;
   bool active = false, tracing = false, exhausted = false;
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, !active);
@@ -441,22 +439,17 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
         if (g < total) {
           J = &A.jobs[find_job(A.jobs, A.njobs, g, false)];
           const uint64_t local = g - J->sample_base;
-          pixel = div_spp(local, J->spp);
-          sample = (uint32_t)(local - (uint64_t)pixel * J->spp);
+          const uint32_t pixel = div_spp(local, J->spp);
           const uint64_t p = J->pixel_base + pixel;
           const float4 r0 = A.cam[2 * p], r1 = A.cam[2 * p + 1];
           const uint32_t bits = __float_as_uint(r1.w);
           if (bits != kDead) {
             sc = &A.scenes[J->scene];
-            st.o = mk(r0.x, r0.y, r0.z);
-            st.d = mk(r1.x, r1.y, r1.z);
+            tr.resume(mk(r0.x, r0.y, r0.z), mk(r1.x, r1.y, r1.z), bits & 0x07FFFFFFu, r0.w, stack);
+            tr.st.set(stack, swrx::kRowUser, make_uint2(pixel, (uint32_t)(local - (uint64_t)pixel * J->spp)));
             st.c = mk(1.0f, 1.0f, 1.0f);
-            st.L = mk(0.0f, 0.0f, 0.0f);
             st.i = bits >> 27;
             st.v = 0;
-            pend_slot = bits & 0x07FFFFFFu;
-            pend_t = r0.w;
-            tr.no_hit(stack);  // the camera record's hit is settled
             tape.reset();
             tracing = false;
             active = true;
@@ -470,12 +463,7 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
     }
     if (active && tracing && tr.step<false, false, swrx::kRuleReference, true, true>(sc->nodes, sc->tris, sc->tri_boxes, sc->obj_boxes, stack, nullptr)) {
       tracing = false;
-      if (tr.hit_slot(stack) == 0xFFFFFFFFu) {  // the path left the scene: no emitter, no gradient
-        active = false;
-      } else {
-        pend_slot = tr.hit_slot(stack);
-        pend_t = tr.hit_t(stack);
-      }
+      if (tr.hit_slot(stack) == 0xFFFFFFFFu) active = false;  // the path left the scene: no emitter, no gradient
     }
     // lanes with a pending hit wait until A.batch of them (or every active lane) shade together
     const unsigned waiting = __ballot_sync(0xffffffffu, active && !tracing);
@@ -487,6 +475,13 @@ __global__ void __launch_bounds__(kTB) k_badjoint(BArgs A, BCtrl* __restrict__ c
       tracing = true;
       continue;
     }
+    const uint32_t pend_slot = tr.hit_slot(stack);
+    const float pend_t = tr.hit_t(stack);
+    const uint2 where = tr.st.get(stack, swrx::kRowUser);
+    const uint32_t pixel = where.x, sample = where.y;
+    st.o = tr.o;
+    st.d = tr.d;
+    st.L = mk(0.0f, 0.0f, 0.0f);
     swrx::ShadeParams P;
     P.seed = J->seed;
     P.pixel = pixel;

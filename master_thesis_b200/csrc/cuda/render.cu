@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kTraceBlock)
             st.v = 0;
             pend_slot = bits & 0x07FFFFFFu;
             pend_t = r0.w;
-            tr.no_hit(stack);  // the camera record's hit is settled
+            tr.st.set(stack, swrx::kRowHit, make_uint2(kDeadSlot, 0u));  // the camera record's hit is settled
             tape.reset();
             tracing = false;
             active = true;
@@ -716,11 +716,9 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
   const unsigned long long total = ctrl->total;
   swrx::Traversal tr;
   tr.setup(stack);
-  uint32_t pixel = 0, sample = 0, phase = kVision, i = 0, draws = 0, vfirst = 0, dv = 0, dl = 0;
+  uint32_t phase = kVision, i = 0, draws = 0, vfirst = 0, dv = 0, dl = 0;
   bool active = false, tracing = false, exhausted = false, vlight = false;
-  f3 o = mk(0, 0, 0), d = mk(0, 0, 0), c = mk(1, 1, 1);
-  uint32_t hslot = 0;
-  float ht = 0.0f;
+  f3 c = mk(1, 1, 1);
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, !active);
     if (!exhausted && (unsigned)__popc(idle) >= F.refill) {
@@ -732,21 +730,17 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       if (!active) {
         const unsigned long long g = base + __popc(idle & lt);
         if (g < total) {
-          pixel = div_spp(F, (uint32_t)g);
-          sample = (uint32_t)g - pixel * F.spp;
+          const uint32_t pixel = div_spp(F, (uint32_t)g), sample = (uint32_t)g - pixel * F.spp;
           const float4 r0 = F.cam[2 * (size_t)pixel], r1 = F.cam[2 * (size_t)pixel + 1];
           const uint32_t bits = __float_as_uint(r1.w);
           if (bits == kDeadSlot) {  // no front hit within visionJumpCount: the sample adds nothing
             F.contrib[(size_t)pixel * F.spp + sample] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             B.head[(size_t)pixel * F.spp + sample] = make_uint4(0u, 0u, 0u, 1u);
           } else {
-            o = mk(r0.x, r0.y, r0.z);
-            d = mk(r1.x, r1.y, r1.z);
+            tr.resume(mk(r0.x, r0.y, r0.z), mk(r1.x, r1.y, r1.z), bits & 0x07FFFFFFu, r0.w, stack);
+            tr.st.set(stack, swrx::kRowUser, make_uint2(pixel, sample));
             i = bits >> 27;
             vfirst = i;
-            hslot = bits & 0x07FFFFFFu;
-            ht = r0.w;
-            tr.no_hit(stack);  // the camera record's hit is settled
             draws = 0;
             dv = dl = 0;
             vlight = false;
@@ -764,8 +758,6 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     }
     if (active && tracing && tr.step<false, false, swrx::kRuleReference, kTriLoop, kTriLoop>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, stack, nullptr)) {
       tracing = false;
-      hslot = tr.hit_slot(stack);
-      ht = tr.hit_t(stack);
     }
     // Lanes whose trace is finished wait until B.batch of them (or every active lane) can run
     // their stage code together, instead of running it for one or two lanes at a time.
@@ -778,6 +770,11 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       tracing = true;
       continue;
     }
+    const uint2 where = tr.st.get(stack, swrx::kRowUser);
+    const uint32_t pixel = where.x, sample = where.y;
+    const uint32_t hslot = tr.hit_slot(stack);
+    const float ht = tr.hit_t(stack);
+    f3 o = tr.o, d = tr.d;
     const uint32_t gpix = F.pixel0 + pixel;
     const uint32_t q = pixel * F.spp + sample;
     // advance the sample until it needs a trace or is finished
@@ -1791,7 +1788,9 @@ int render_bdpt_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts*
   B.vtx = (float4*)ws->bd_vtx;
   B.head = (uint4*)ws->bd_head;
   const bool few = s->dev.num_tris <= swrx::kFewTriangles;
-  auto kern = few ? k_bdpt_paths<0, true> : k_bdpt_paths<0, false>;
+  // 5 blocks per SM (96 registers); left to itself the compiler takes 114 registers and 4 blocks, 6 % slower
+  // on a 200,000-triangle model
+  auto kern = few ? k_bdpt_paths<5, true> : k_bdpt_paths<5, false>;
   auto kconn = few ? k_bdpt_connect<0, true> : k_bdpt_connect<0, false>;
   if (b->blocks_per_sm == 5) kern = k_bdpt_paths<5, false>, kconn = k_bdpt_connect<5, false>;
   else if (b->blocks_per_sm == 6) kern = k_bdpt_paths<6, false>, kconn = k_bdpt_connect<6, false>;

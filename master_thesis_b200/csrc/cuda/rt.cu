@@ -60,47 +60,60 @@ __device__ __forceinline__ void store_pixel(const RtFrame& F, uint32_t p, f3 c) 
   if (F.rgba) F.rgba[p] = make_uchar4(rt::unorm8(c.x), rt::unorm8(c.y), rt::unorm8(c.z), 0);
 }
 
-// The first hit's payload of each lane's pixel (the raygen's defaultRayPayload), read back at the
-// start of every sample: kept in shared memory, one column per thread, instead of 12 registers.
-struct DefPayload {
-  float v[12][kBlock];
-  __device__ void put(const rt::Payload& P) {
-    const float a[12] = {P.pos.x, P.pos.y, P.pos.z, P.n.x, P.n.y, P.n.z, P.color.x, P.color.y, P.color.z,
-                         P.dT, P.rT, P.tT};
-#pragma unroll
-    for (int k = 0; k < 12; ++k) v[k][threadIdx.x] = a[k];
+// What a lane's pixel keeps between its rays' shadings: the first hit's payload (the raygen's
+// defaultRayPayload) and the pixel's own ray direction, read back at the start of every sample, the
+// sum so far, the sample's colour, and the pixel and sample. In shared memory, one column per
+// thread: none of it is used while a ray is traced.
+struct PixelState {
+  float v[22][kBlock];
+  uint32_t n[2][kBlock];
+  __device__ void put3(int k, f3 a) {
+    v[k][threadIdx.x] = a.x;
+    v[k + 1][threadIdx.x] = a.y;
+    v[k + 2][threadIdx.x] = a.z;
   }
-  __device__ rt::Payload get(float eta) const {
+  __device__ f3 get3(int k) const { return mk(v[k][threadIdx.x], v[k + 1][threadIdx.x], v[k + 2][threadIdx.x]); }
+  __device__ void put(const rt::Payload& P) {
+    put3(0, P.pos);
+    put3(3, P.n);
+    put3(6, P.color);
+    const float a[4] = {P.dT, P.rT, P.tT, P.eta};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[9 + k][threadIdx.x] = a[k];
+  }
+  __device__ rt::Payload get() const {
     rt::Payload P;
     const unsigned t = threadIdx.x;
-    P.pos = mk(v[0][t], v[1][t], v[2][t]);
-    P.n = mk(v[3][t], v[4][t], v[5][t]);
-    P.color = mk(v[6][t], v[7][t], v[8][t]);
+    P.pos = get3(0);
+    P.n = get3(3);
+    P.color = get3(6);
     P.dT = v[9][t];
     P.rT = v[10][t];
     P.tT = v[11][t];
-    P.eta = eta;
+    P.eta = v[12][t];
     P.light = 0u;  // a first hit on a light ends the pixel before any sample
     return P;
   }
 };
+enum { kDirection = 13, kSum = 16, kColor = 19 };  // rows of PixelState::v
+enum { kPixel = 0, kSample = 1 };                  // rows of PixelState::n
 
-// kMinBlocks: resident blocks per SM the register budget targets (0 = the compiler's choice)
+// kMinBlocks: resident blocks per SM the register budget targets (0: the compiler's choice, 72
+// registers and 7 blocks; with the pixel's state in registers it was 80 and 6 blocks, the RayTrace
+// frame 5.00 instead of 4.81 ms)
 template <int kMinBlocks, bool kTriLoop>
 __global__ void __launch_bounds__(kBlock, kMinBlocks)
     k_rt_path(DevScene sc, RtFrame F, unsigned long long* __restrict__ cursor) {
   __shared__ __align__(1024) uint2 stack[swrx::kTraceMem * kBlock];
-  __shared__ DefPayload defs;
+  __shared__ PixelState px;
+  const unsigned tid = threadIdx.x;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
   const unsigned long long total = (unsigned long long)F.W * F.H;
   swrx::Traversal tr;
   tr.setup(stack);
-  rt::Payload cur;
-  float def_eta = 0.0f;
-  uint32_t pixel = 0, rng = 0, s = 0, i = 0, cull = 0, stage = kPrimary;
+  uint32_t rng = 0, i = 0, stage = kPrimary;  // i: the retries so far while the stage is kPrimary
   bool active = false, tracing = false, exhausted = false;
-  f3 o = mk(0, 0, 0), d = mk(0, 0, 0), sdir = mk(0, 0, 0), col = mk(0, 0, 0), fin = mk(0, 0, 0);
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, !active);
     if (!exhausted && (unsigned)__popc(idle) >= F.refill) {
@@ -111,13 +124,15 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
       if (!active) {
         const unsigned long long g = base + __popc(idle & lt);
         if (g < total) {
-          pixel = (uint32_t)g;
+          const uint32_t pixel = (uint32_t)g;
           const uint32_t x = pixel % F.W, y = pixel / F.W;
           rng = rt::lcg_init(x, y, 0u);
+          f3 o, d;
           rt::vision_ray(F.vi, F.pi, x, y, F.W, F.H, o, d);
-          sdir = d;
-          cull = 0;
-          fin = mk(0.0f, 0.0f, 0.0f);
+          px.n[kPixel][tid] = pixel;
+          px.put3(kDirection, d);
+          px.put3(kSum, mk(0.0f, 0.0f, 0.0f));
+          i = 0;
           stage = kPrimary;
           tr.init(o, d, stack);
           tracing = true;
@@ -139,31 +154,35 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
     if (waiting == 0u || ((unsigned)__popc(waiting) < F.shade_batch && inflight != 0u)) continue;
     if (!active || tracing) continue;
     const uint32_t hs = tr.hit_slot(stack);
+    f3 o = tr.o, d = tr.d;
+    f3 col;
+    rt::Payload cur;
+    uint32_t s;
     if (stage == kPrimary) {
       // traceRay with back-face culling: up to four traces, each retry from the culled hit
       if (hs == kMiss) {
-        store_pixel(F, pixel, mk(0.0f, 0.0f, 0.0f));
+        store_pixel(F, px.n[kPixel][tid], mk(0.0f, 0.0f, 0.0f));
         active = false;
         continue;
       }
       const rt::Payload P = rt::hit_payload(sc.tris, sc.shade, sc.mats, hs, o, d);
-      if (swrx::vdot(P.n, d) > 0.0f && cull < 3) {
-        o = P.pos;
-        ++cull;
-        tr.init(o, d, stack);
+      if (swrx::vdot(P.n, d) > 0.0f && i < 3) {
+        ++i;
+        tr.init(P.pos, d, stack);
         tracing = true;
         continue;
       }
       if (P.light) {  // a light seen directly: its color * lightStrength, unscaled
-        store_pixel(F, pixel, P.color);
+        store_pixel(F, px.n[kPixel][tid], P.color);
         active = false;
         continue;
       }
-      defs.put(P);
-      def_eta = P.eta;
+      px.put(P);
       s = 0;
       stage = kSampleStart;
     } else {  // kJumpResult
+      s = px.n[kSample][tid];
+      col = px.get3(kColor);
       if (hs == kMiss) {  // color = 0: the sample adds nothing
         ++s;
         stage = kSampleStart;
@@ -171,7 +190,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
         const rt::Payload P = rt::hit_payload(sc.tris, sc.shade, sc.mats, hs, o, d);
         if (P.light && swrx::vdot(d, P.n) <= 0.0f) {
           col = swrx::vmul(col, P.color);
-          fin = swrx::vadd(fin, col);
+          px.put3(kSum, swrx::vadd(px.get3(kSum), col));
           ++s;
           stage = kSampleStart;
         } else {
@@ -185,12 +204,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
     while (!tracing) {
       if (stage == kSampleStart) {
         if (s >= F.spp) {
-          store_pixel(F, pixel, swrx::vscale(F.scale, fin));
+          store_pixel(F, px.n[kPixel][tid], swrx::vscale(F.scale, px.get3(kSum)));
           active = false;
           break;
         }
-        cur = defs.get(def_eta);
-        d = sdir;
+        cur = px.get();
+        d = px.get3(kDirection);
         col = mk(1.0f, 1.0f, 1.0f);
         i = 1;
         stage = kJump;
@@ -206,6 +225,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
                                  swrx::fmul(cur.color.z, cs)));
       }
       tr.init(o, d, stack);
+      px.n[kSample][tid] = s;
+      px.put3(kColor, col);
       tracing = true;
       stage = kJumpResult;
     }
@@ -392,13 +413,22 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_rt_opts* opts, fl
   unsigned long long* cursor = (unsigned long long*)s->d_scratch;
   SWR_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
   const bool few = s->dev.num_tris <= swrx::kFewTriangles;
-  auto kern = few ? k_rt_path<0, true> : k_rt_path<0, false>;
-  if (opts->blocks_per_sm == 5) kern = few ? k_rt_path<5, true> : k_rt_path<5, false>;
-  else if (opts->blocks_per_sm == 6) kern = few ? k_rt_path<6, true> : k_rt_path<6, false>;
+  // Resident blocks per SM: a pixel's samples follow one another on its lane, so an image of about as
+  // many pixels as the GPU has lanes takes as long as its longest pixel, and fewer blocks that each
+  // run faster win. 230,400 pixels at 7 / 5 blocks: a 30,000-triangle model 1.36 / 1.16 ms, a terrain of
+  // 0.5 M triangles 2.30 / 2.16, Cornell 0.81 / 0.86; 2 M pixels: 5.53 / 5.97, 6.06 / 6.42, 4.80 / 5.35.
+  // Between them large scenes, whose pixels differ most, take 6 (921,600 pixels of the terrain: 3.34,
+  // 7 blocks 3.49).
+  const uint64_t npix = (uint64_t)F.W * F.H;
+  uint32_t blocks = opts->blocks_per_sm;
+  if (blocks == 0)
+    blocks = npix <= (1u << 18) ? 5 : (npix < (1u << 20) && s->dev.num_tris > (1u << 16)) ? 6 : 7;
+  auto kern = few ? k_rt_path<0, true> : k_rt_path<0, false>;  // 72 registers: 7 blocks
+  if (blocks == 5) kern = few ? k_rt_path<5, true> : k_rt_path<5, false>;
+  else if (blocks == 6) kern = few ? k_rt_path<6, true> : k_rt_path<6, false>;
   int per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0));
   per_sm = std::max(per_sm, 1);
-  const uint64_t npix = (uint64_t)F.W * F.H;
   const uint64_t need = (npix + kBlock - 1) / kBlock;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)s->num_sms * per_sm, need));
   kern<<<grid, kBlock, 0, stream>>>(s->dev, F, cursor);

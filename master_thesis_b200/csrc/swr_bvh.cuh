@@ -313,8 +313,14 @@ struct Traversal {
 
   SWR_HD uint32_t hit_slot(const uint2* mem) const { return st.get(mem, kRowHit).x; }
   SWR_HD float hit_t(const uint2* mem) const { return bits2f(st.get(mem, kRowHit).y); }
-  // the ray counts as settled without a hit (a lane that starts from a stored hit)
-  SWR_HD void no_hit(uint2* mem) { st.set(mem, kRowHit, make_uint2(0xFFFFFFFFu, 0u)); }
+  // A finished, settled ray made from a stored hit (a sample that starts at its camera record): the
+  // kernels whose lanes wait for one another between rays keep nothing of a ray but this object.
+  SWR_HD void resume(f3 o_, f3 d_, uint32_t slot, float t, uint2* mem) {
+    o = o_;
+    d = d_;
+    st.set(mem, kRowHit, make_uint2(slot, f2bits(t)));
+    st.set(mem, kRowDist, make_uint2(0u, kStrict));
+  }
 
   // Whether a finished ray's hit stands: always for a miss (no candidate at all) and after a strict
   // pass; otherwise when the hit triangle's and its object's reference boxes pass the slab test.
