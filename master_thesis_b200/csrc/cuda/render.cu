@@ -34,11 +34,12 @@ constexpr uint32_t kDeadSlot = 0xFFFFFFFFu;
 constexpr int kTraceBlock = swrx::kTraceThreads;
 constexpr uint64_t kChunkSamples = 1ull << 27;
 // chunks of at least this many samples, on scenes of at least kTwoWaveTriangles triangles, run as
-// kSubWaves concurrent sub-wavefronts (SWR_RENDER_ONE_WAVEFRONT). Measured on B200: 28.02 vs 28.49
-// ms for the 2.4 M-triangle terrain image; 1-2 % slower on the 36-triangle Cornell box, whose
-// traversal launches have no long tail to fill.
+// kSubWaves concurrent sub-wavefronts (SWR_RENDER_ONE_WAVEFRONT): 8.4 M samples of the 47,000-triangle
+// tessellated Cornell box 6.9 -> 6.5 ms, the 2.4 M-triangle terrain image 20.6 (sum of its kernels) ->
+// 19.0 ms; 36 to 30,000 triangles, whose traversal launches have no long tail to fill, within 2 % or
+// slower.
 constexpr uint64_t kTwoWaveSamples = 1ull << 20;
-constexpr uint32_t kTwoWaveTriangles = 1u << 16;
+constexpr uint32_t kTwoWaveTriangles = 1u << 15;
 constexpr int kSubWaves = 2;
 
 struct Ctrl {
