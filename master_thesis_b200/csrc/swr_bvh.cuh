@@ -204,6 +204,18 @@ SWR_HD float fmax3_relu(float a, float b, float c) {
   return fmaxf(fmaxf(a, b), fmaxf(c, 0.0f));
 #endif
 }
+// (x0, y0) = (a0 * b0 + c0, a1 * b1 + c1), each rounded once: one instruction for both on the device
+SWR_HD void fma2(float a0, float a1, float b0, float b1, float c0, float c1, float& x0, float& x1) {
+#if defined(__CUDA_ARCH__)
+  asm("{.reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+      " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;}"
+      : "=f"(x0), "=f"(x1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+#else
+  x0 = fmaf(a0, b0, c0);
+  x1 = fmaf(a1, b1, c1);
+#endif
+}
 // m shifted left by one with x's sign let in
 SWR_HD uint32_t push_sign(uint32_t m, float x) {
 #if defined(__CUDA_ARCH__)
@@ -477,8 +489,11 @@ struct Traversal {
         const float qfx = plane_level(i < 4 ? fx0 : fx1, i & 3);
         const float qfy = plane_level(i < 4 ? fy0 : fy1, i & 3);
         const float qfz = plane_level(i < 4 ? fz0 : fz1, i & 3);
-        const float tnx = fmaf(qnx, ax, bx), tny = fmaf(qny, ay, by), tnz = fmaf(qnz, az, bz);
-        const float tfx = fmaf(qfx, ax, bx), tfy = fmaf(qfy, ay, by), tfz = fmaf(qfz, az, bz);
+        float tnx, tny, tnz, tfx, tfy, tfz;
+        fma2(qnx, qny, ax, ay, bx, by, tnx, tny);
+        fma2(qfx, qfy, ax, ay, bx, by, tfx, tfy);
+        tnz = fmaf(qnz, az, bz);
+        tfz = fmaf(qfz, az, bz);
         const float tn = fmax3_relu(tnx, tny, tnz);
         const float tf = fmin3(tfx, tfy, fminf(tfz, tprune));
         miss = push_sign(miss, fsub(tf, tn));
