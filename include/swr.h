@@ -330,7 +330,7 @@ int swr_scene_set_emission(swr_scene* scene, const float* emission, void* stream
 
 /* swr_scene_set_albedo and swr_scene_set_emission of many scenes in one launch (inverse rendering
  * sets every scene of a batch before each pass). The scenes differ from each other and are on the
- * batch's device. */
+ * batch's device. Refused while the stream is being captured (the per-scene calls are not). */
 typedef struct swr_parameter_job {
   swr_scene* scene;
   const float* albedo;

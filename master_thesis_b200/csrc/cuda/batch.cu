@@ -895,6 +895,11 @@ int swr_batch_set_parameters(swr_batch* b, const swr_parameter_job* jobs, uint32
   if (!b || !jobs || n == 0) return set_error(SWR_ERR_INVALID, "swr: empty batch");
   cudaStream_t stream = (cudaStream_t)stream_;
   SWR_CUDA(cudaSetDevice(b->device));
+  // a graph would keep the address of the job table built below, which ends with this call
+  cudaStreamCaptureStatus capture;
+  SWR_CUDA(cudaStreamIsCapturing(stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone)
+    return set_error(SWR_ERR_UNSUPPORTED, "swr: swr_batch_set_parameters cannot be captured");
   bool staged = false;  // host buffers take the per-scene calls, which stage them
   for (uint32_t k = 0; k < n; ++k) {
     if (!jobs[k].scene || !jobs[k].albedo || !jobs[k].emission) return set_error(SWR_ERR_INVALID, "swr: null argument");

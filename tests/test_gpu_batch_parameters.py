@@ -34,3 +34,19 @@ def test_batch_parameters_as_per_scene(where):
     assert lit > 0
     with pytest.raises(swr.SwrError if hasattr(swr, "SwrError") else Exception):
         batch.set_parameters([], [], [])
+
+
+def test_batch_parameters_refused_under_capture():
+    import torch
+    d = scenes.random_scene(7, 64)[0]
+    scene, batch = swr.Scene(d), swr.Batch()
+    alb = torch.full((d.num_triangles, 3), 0.5, device="cuda")
+    em = torch.ones((d.num_objects, 3), device="cuda")
+    batch.set_parameters([scene], [alb], [em])
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        with pytest.raises(Exception, match="captured"):
+            batch.set_parameters([scene], [alb], [em], stream=torch.cuda.current_stream())
+        alb.add_(0.0)
+    g.replay()
+    torch.cuda.synchronize()
