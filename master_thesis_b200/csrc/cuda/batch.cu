@@ -614,6 +614,7 @@ struct swr_batch {
   std::vector<char> graph_key[4];
   cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // streams of sub-wavefronts 1..3
   cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t params_read = nullptr;  // after the last launch that reads params
   int device = -1;
 };
 
@@ -663,6 +664,17 @@ int add_job(int device, const swr_scene* scene, const swr_camera& cam, const swr
   return SWR_OK;
 }
 
+// Copies a table of jobs to b->params once the launch that read the last one, on whichever stream, is
+// through with it.
+int put_params(swr_batch* b, const void* table, size_t bytes, cudaStream_t stream) {
+  if (b->params_read) SWR_CUDA(cudaStreamWaitEvent(stream, b->params_read, 0));
+  else SWR_CUDA(cudaEventCreateWithFlags(&b->params_read, cudaEventDisableTiming));
+  int rc;
+  if ((rc = ensure_bytes(&b->params, b->parambytes, bytes))) return rc;
+  SWR_CUDA(cudaMemcpyAsync(b->params, table, bytes, cudaMemcpyHostToDevice, stream));
+  return SWR_OK;
+}
+
 }  // namespace
 }  // namespace swr
 
@@ -686,6 +698,7 @@ void swr_batch_destroy(swr_batch* b) {
     if (b->join[h]) cudaEventDestroy(b->join[h]);
   }
   if (b->fork) cudaEventDestroy(b->fork);
+  if (b->params_read) cudaEventDestroy(b->params_read);
   for (void* p : {b->qbuf, b->cam, b->accum, b->jobs, b->scenes, b->ctrl, b->params})
     if (p) cudaFree(p);
   if (b->host_ctrl) cudaFreeHost(b->host_ctrl);
@@ -925,10 +938,10 @@ int swr_batch_set_parameters(swr_batch* b, const swr_parameter_job* jobs, uint32
       blocks += (nt + kParamBlock - 1) / kParamBlock + (no + kParamBlock - 1) / kParamBlock;
     }
     if (blocks > 0x7FFFFFFFull) return set_error(SWR_ERR_UNSUPPORTED, "swr: too many triangles in one call");
-    if ((rc = ensure_bytes(&b->params, b->parambytes, n * sizeof(ParamJob)))) return rc;
-    SWR_CUDA(cudaMemcpyAsync(b->params, hp.data(), n * sizeof(ParamJob), cudaMemcpyHostToDevice, stream));
+    if ((rc = put_params(b, hp.data(), n * sizeof(ParamJob), stream))) return rc;
     k_set_parameters<<<(unsigned)blocks, kParamBlock, 0, stream>>>((const ParamJob*)b->params, n);
     SWR_CUDA(cudaGetLastError());
+    SWR_CUDA(cudaEventRecord(b->params_read, stream));
   } catch (const std::bad_alloc&) {
     return set_error(SWR_ERR_ALLOC, "swr: host allocation failed");
   }
@@ -991,14 +1004,14 @@ int swr_render_adjoint_batch(swr_batch* b, const swr_adjoint_job* jobs, uint32_t
   // at most 65535 buffers (the grid's second dimension) per launch
   std::vector<ZeroJob> hz;
   for (auto& z : zero) hz.push_back({z.first, z.second / sizeof(float)});
-  if ((rc = ensure_bytes(&b->params, b->parambytes, hz.size() * sizeof(ZeroJob)))) return rc;
-  SWR_CUDA(cudaMemcpyAsync(b->params, hz.data(), hz.size() * sizeof(ZeroJob), cudaMemcpyHostToDevice, stream));
+  if ((rc = put_params(b, hz.data(), hz.size() * sizeof(ZeroJob), stream))) return rc;
   for (size_t z0 = 0; z0 < hz.size(); z0 += 65535) {
     const unsigned nz = (unsigned)std::min<size_t>(65535, hz.size() - z0);
     const unsigned per = std::max(1u, (unsigned)(num_sms * 8) / nz);
     k_zero<<<dim3(per, nz), 256, 0, stream>>>((const ZeroJob*)b->params + z0);
     SWR_CUDA(cudaGetLastError());
   }
+  SWR_CUDA(cudaEventRecord(b->params_read, stream));
   BArgs A;
   std::memset(&A, 0, sizeof(A));
   A.jobs = (const BJob*)b->jobs;

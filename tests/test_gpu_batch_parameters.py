@@ -50,3 +50,29 @@ def test_batch_parameters_refused_under_capture():
         alb.add_(0.0)
     g.replay()
     torch.cuda.synchronize()
+
+
+def test_batch_parameters_from_two_streams():
+    """The second call's table is not written before the first call's launch has read its own."""
+    import torch
+    datas = [scenes.random_scene(60 + k, 256)[0] for k in range(2)]
+    alb = [torch.rand((d.num_triangles, 3), generator=torch.Generator().manual_seed(k)).cuda()
+           for k, d in enumerate(datas)]
+    em = [torch.full((d.num_objects, 3), 2.0 + k, device="cuda") for k, d in enumerate(datas)]
+    W, H = 24, 16
+    cam = swr.make_camera((4.0, 2.5, 4.0), (-0.75, -0.3), W, H, fov_deg=60.0)
+    one, many = [swr.Scene(d) for d in datas], [swr.Scene(d) for d in datas]
+    batch = swr.Batch()
+    streams = [torch.cuda.Stream() for _ in datas]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(20_000_000)  # the first launch waits about 10 ms
+    for k in range(2):
+        batch.set_parameters([many[k]], [alb[k]], [em[k]], stream=streams[k])
+    torch.cuda.synchronize()
+    for k in range(2):
+        one[k].set_albedo(alb[k])
+        one[k].set_emission(em[k])
+        x = one[k].render(cam, W, H, 64, 4, seed=1, mode=swr.MODE_PHYSICAL)
+        assert torch.count_nonzero(x) > 0
+        assert torch.equal(x, many[k].render(cam, W, H, 64, 4, seed=1, mode=swr.MODE_PHYSICAL))
