@@ -1274,6 +1274,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   KernelTimer timer;
   timer.on = (o->flags & SWR_RENDER_PROFILE) != 0;
   const bool count = (o->flags & SWR_RENDER_COUNT) != 0;
+  const bool host_loop = timer.on || (o->flags & SWR_RENDER_HOST_LOOP) != 0;
 
   // the pixels this call renders (the whole image unless a pixel range is given)
   const uint64_t npix_total = part.npix;
@@ -1472,7 +1473,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     F.npix = np;
     const uint64_t total = (uint64_t)np * o->spp;
     SWR_CUDA(cudaStreamSynchronize(stream));  // the pinned control blocks may still be in flight
-    if (!timer.on && !(o->flags & SWR_RENDER_HOST_LOOP)) {
+    if (!host_loop) {
       // Large chunks of large scenes run as kSubWaves sub-wavefronts (a share of the pixels and of
       // the paths in flight each) on as many streams: when one's traversal launch runs out of rays and its SMs
       // idle while the last rays finish, the others' kernels fill them. Per-pixel results do not
@@ -1578,7 +1579,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       if (host_samples) P.d2h_bytes += bytes;
     }
   }
-  if (host_img && timer.on) {  // the graph path copied each sub-wavefront's part as it finished
+  if (host_img && host_loop) {  // the graph path copied each sub-wavefront's part as it finished
     SWR_CUDA(cudaMemcpyAsync(rgb_out, img_dev, npix_total * 3 * sizeof(float), cudaMemcpyDeviceToHost, stream));
     P.d2h_bytes += npix_total * 3 * sizeof(float);
   }
