@@ -329,8 +329,9 @@ int swr_scene_set_albedo(swr_scene* scene, const float* albedo, void* stream);
 int swr_scene_set_emission(swr_scene* scene, const float* emission, void* stream);
 
 /* swr_scene_set_albedo and swr_scene_set_emission of many scenes in one launch (inverse rendering
- * sets every scene of a batch before each pass). The scenes differ from each other and are on the
- * batch's device. Refused while the stream is being captured (the per-scene calls are not). */
+ * sets every scene of a batch before each pass). The scenes are on the batch's device. A list that
+ * names a scene twice, or a buffer in host memory, is set entry by entry in the list's order. Refused
+ * while the stream is being captured (the per-scene calls are not). */
 typedef struct swr_parameter_job {
   swr_scene* scene;
   const float* albedo;

@@ -358,7 +358,11 @@ class Batch:
         return outs
 
     def set_parameters(self, scenes, albedos, emissions, stream=None):
-        """Scene.set_albedo and Scene.set_emission of many scenes (each once) in one launch."""
+        """Scene.set_albedo and Scene.set_emission of many scenes in one launch (a scene named twice
+        keeps its last entry)."""
+        if not len(scenes) == len(albedos) == len(emissions):
+            raise ValueError("set_parameters: %d scenes, %d albedos, %d emissions" %
+                             (len(scenes), len(albedos), len(emissions)))
         arr = (N.ParameterJob * len(scenes))()
         for k, sc in enumerate(scenes):
             arr[k].scene, arr[k].albedo, arr[k].emission = sc.handle, ptr(albedos[k]), ptr(emissions[k])

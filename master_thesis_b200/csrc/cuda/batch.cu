@@ -913,21 +913,28 @@ int swr_batch_set_parameters(swr_batch* b, const swr_parameter_job* jobs, uint32
   SWR_CUDA(cudaStreamIsCapturing(stream, &capture));
   if (capture != cudaStreamCaptureStatusNone)
     return set_error(SWR_ERR_UNSUPPORTED, "swr: swr_batch_set_parameters cannot be captured");
-  bool staged = false;  // host buffers take the per-scene calls, which stage them
-  for (uint32_t k = 0; k < n; ++k) {
-    if (!jobs[k].scene || !jobs[k].albedo || !jobs[k].emission) return set_error(SWR_ERR_INVALID, "swr: null argument");
-    if (jobs[k].scene->device != b->device) return set_error(SWR_ERR_INVALID, "swr: batch jobs on another device");
-    staged = staged || is_host_pointer(jobs[k].albedo) || is_host_pointer(jobs[k].emission);
-  }
   int rc;
-  if (staged) {
-    for (uint32_t k = 0; k < n; ++k) {
-      if ((rc = swr_scene_set_albedo(jobs[k].scene, jobs[k].albedo, stream_))) return rc;
-      if ((rc = swr_scene_set_emission(jobs[k].scene, jobs[k].emission, stream_))) return rc;
-    }
-    return SWR_OK;
-  }
   try {
+    // The per-scene calls, in order: for host buffers, which they stage, and for a list that names a
+    // scene twice, whose blocks would write it in any order within one launch (the last entry holds).
+    bool one_by_one = false;
+    std::vector<const swr_scene*> named(n);
+    for (uint32_t k = 0; k < n; ++k) {
+      if (!jobs[k].scene || !jobs[k].albedo || !jobs[k].emission)
+        return set_error(SWR_ERR_INVALID, "swr: null argument");
+      if (jobs[k].scene->device != b->device) return set_error(SWR_ERR_INVALID, "swr: batch jobs on another device");
+      one_by_one = one_by_one || is_host_pointer(jobs[k].albedo) || is_host_pointer(jobs[k].emission);
+      named[k] = jobs[k].scene;
+    }
+    std::sort(named.begin(), named.end());
+    one_by_one = one_by_one || std::adjacent_find(named.begin(), named.end()) != named.end();
+    if (one_by_one) {
+      for (uint32_t k = 0; k < n; ++k) {
+        if ((rc = swr_scene_set_albedo(jobs[k].scene, jobs[k].albedo, stream_))) return rc;
+        if ((rc = swr_scene_set_emission(jobs[k].scene, jobs[k].emission, stream_))) return rc;
+      }
+      return SWR_OK;
+    }
     std::vector<ParamJob> hp(n);
     uint64_t blocks = 0;
     for (uint32_t k = 0; k < n; ++k) {

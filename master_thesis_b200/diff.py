@@ -52,7 +52,8 @@ class _PhysicalRenderBatch(torch.autograd.Function):
     @staticmethod
     def forward(ctx, batch, jobs, adjoint_seeds, *params):
         params = [p.detach().contiguous() for p in params]
-        batch.set_parameters([j["scene"] for j in jobs], params[0::2], params[1::2])
+        n = 2 * len(jobs)
+        batch.set_parameters([j["scene"] for j in jobs], params[0:n:2], params[1:n:2])
         imgs = batch.render([dict(j, mode=N.MODE_PHYSICAL) for j in jobs])
         ctx.save_for_backward(*params)
         ctx.batch, ctx.jobs, ctx.adjoint_seeds = batch, jobs, adjoint_seeds
@@ -62,7 +63,8 @@ class _PhysicalRenderBatch(torch.autograd.Function):
     def backward(ctx, *grads):
         params = ctx.saved_tensors
         adj = []
-        ctx.batch.set_parameters([j["scene"] for j in ctx.jobs], params[0::2], params[1::2])
+        n = 2 * len(ctx.jobs)
+        ctx.batch.set_parameters([j["scene"] for j in ctx.jobs], params[0:n:2], params[1:n:2])
         for k, j in enumerate(ctx.jobs):
             g = grads[k]
             if g is None:
