@@ -985,7 +985,12 @@ __global__ void k_dark_samples(float4* __restrict__ contrib, uint64_t n, float f
 // 2.1 GB of slots is their few lit ones. The loads are coalesced (neighbouring lanes read
 // neighbouring slots of a pixel) into a shared-memory tile padded to 9 slots per pixel
 // (conflict-free reads); each lane then adds its pixel's slots in sample order, as the reference's
-// renderPixel does.
+// renderPixel does. An image of few pixels with many samples is one serial chain of groups: what a
+// group takes is the latency of its slots, as long as neither the next bits (loaded a word ahead) nor
+// the reads of the tile (all eight before the sums, dark slots as zeros that are not added) wait in
+// line behind it. One pixel of 262,144 lit samples: 33.8 ms with the bits walked one by one, 22.1
+// without any bits, 21.1 so; 64x64 pixels of 2,048 samples 1.07, 0.84 and 0.79 ms. The terrain image's
+// sums take 93 us (104 with the bits walked).
 __global__ void __launch_bounds__(256) k_resolve(Frame F, float* __restrict__ img) {
   __shared__ float4 tile[8][32 * 9];
   const uint32_t w = threadIdx.x >> 5, lane = lane_id();
@@ -996,31 +1001,42 @@ __global__ void __launch_bounds__(256) k_resolve(Frame F, float* __restrict__ im
   float4* t = tile[w];
   float r = 0.0f, g = 0.0f, b = 0.0f;
   const uint32_t words = lit_words_of(spp);
+  const uint32_t* lit = F.lit ? F.lit + (size_t)(p0 + (lane < np ? lane : 0u)) * words : nullptr;
+  uint32_t next = lit ? lit[0] : 0xFFFFFFFFu;
   for (uint32_t k = 0; k < words; ++k) {
-    uint32_t bits = lane < np ? 0xFFFFFFFFu : 0u;
-    if (F.lit && lane < np) bits = F.lit[(size_t)(p0 + lane) * words + k];
+    uint32_t bits = lane < np ? next : 0u;
+    if (lit && k + 1 < words) next = lit[k + 1];
     if (!__any_sync(0xffffffffu, bits != 0u)) continue;
     const uint32_t left = spp - 32u * k;  // samples from this word on
     if (left < 32u) bits &= (1u << left) - 1u;
     for (uint32_t s0 = 0; s0 < 32u && s0 < left; s0 += 8) {
       const uint32_t mine = (bits >> s0) & 0xFFu;
       if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+      float4 v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint32_t e = lane + 32u * j, pe = e >> 3, se = e & 7u;
         const uint32_t theirs = __shfl_sync(0xffffffffu, mine, pe);
-        if ((theirs >> se) & 1u) t[pe * 9 + se] = __ldcs(F.contrib + (size_t)(p0 + pe) * spp + 32u * k + s0 + se);
+        v[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if ((theirs >> se) & 1u) v[j] = __ldcs(F.contrib + (size_t)(p0 + pe) * spp + 32u * k + s0 + se);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t e = lane + 32u * j;
+        t[(e >> 3) * 9 + (e & 7u)] = v[j];
       }
       __syncwarp();
-      for (uint32_t m = mine; m; m &= m - 1u) {
-        const float4 v = t[lane * 9 + __ffs(m) - 1];
-        if (v.w != 0.0f) {
-          r = __fadd_rn(r, v.x);
-          g = __fadd_rn(g, v.y);
-          b = __fadd_rn(b, v.z);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = t[lane * 9 + j];
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (v[j].w != 0.0f) {
+          r = __fadd_rn(r, v[j].x);
+          g = __fadd_rn(g, v[j].y);
+          b = __fadd_rn(b, v[j].z);
         }
       }
-      __syncwarp();
     }
   }
   if (lane >= np) return;
