@@ -119,6 +119,20 @@ constexpr uint32_t kLitClearedByCamera = 32;
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
+// ORs a sample's bit into its word. A warp's lit samples are often neighbours of one pixel (every
+// sample of a light seen directly): they then share one atomic instead of queueing for the word
+// (256x256 pixels of 256 such samples: 0.42 -> 0.37 ms).
+__device__ __forceinline__ void set_lit(uint32_t* lit, uint64_t word, uint32_t bit) {
+  const unsigned lanes = __activemask();
+  const int first = __ffs(lanes) - 1;
+  if (__all_sync(lanes, word == __shfl_sync(lanes, word, first))) {
+    bit = __reduce_or_sync(lanes, bit);
+    if ((int)lane_id() == first) atomicOr(lit + word, bit);
+  } else {
+    atomicOr(lit + word, bit);
+  }
+}
+
 // Pixel k's camera record; its samples start dark.
 __device__ __forceinline__ void put_camera_record(const Frame& F, uint32_t k, float4 rec0, float4 rec1) {
   F.cam[2 * (size_t)k] = rec0;
@@ -365,7 +379,7 @@ __global__ void __launch_bounds__(kBlock)
           // (an emitter seen from behind, physical mode: a zero adds nothing)
           if (F.mode == 0 || ((__float_as_uint(r.x) | __float_as_uint(r.y) | __float_as_uint(r.z)) << 1) != 0u) {
             __stcs(F.contrib + (size_t)e.pixel * F.spp + e.sample, make_float4(r.x, r.y, r.z, 1.0f));
-            atomicOr(F.lit + (size_t)e.pixel * F.lit_words + (e.sample >> 5), 1u << (e.sample & 31u));
+            set_lit(F.lit, (uint64_t)e.pixel * F.lit_words + (e.sample >> 5), 1u << (e.sample & 31u));
           }
         }
       }
