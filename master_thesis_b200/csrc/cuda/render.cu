@@ -40,6 +40,13 @@ constexpr uint64_t kChunkSamples = 1ull << 27;
 // slower.
 constexpr uint64_t kTwoWaveSamples = 1ull << 20;
 constexpr uint32_t kTwoWaveTriangles = 1u << 15;
+// With a small wave_size, each launch takes as long as its longest ray, and two queues of half the
+// size need twice the launches: scenes of fewer than 2^16 triangles stay one wavefront then (8.4 M
+// samples, 2^16 paths in flight, one / two: 33,000 triangles 15.4 / 17.7 ms, 40,000 17.3 / 20.9, 60,000
+// 21.7 / 23.2, the tessellated Cornell box 46.0 / 44.5; 2^17 paths: 9.0 / 9.8, 10.0 / 11.6, 12.7 / 13.0
+// and 27.1 / 25.3; 2^18 paths: 6.3 / 6.0, 7.1 / 7.1, 9.0 / 8.1 and 17.5 / 15.7).
+constexpr uint32_t kTwoWavePaths = 1u << 17;
+constexpr uint32_t kTwoWaveAnyPaths = 1u << 16;  // triangles
 constexpr int kSubWaves = 2;
 
 struct Ctrl {
@@ -1515,7 +1522,8 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       // idle while the last rays finish, the others' kernels fill them. Per-pixel results do not
       // depend on it.
       const int nsub = (!(o->flags & SWR_RENDER_ONE_WAVEFRONT) && total >= kTwoWaveSamples &&
-                        s->dev.num_tris >= kTwoWaveTriangles && np >= (uint32_t)kSubWaves &&
+                        s->dev.num_tris >= kTwoWaveTriangles &&
+                        (cap >= kTwoWavePaths || s->dev.num_tris >= kTwoWaveAnyPaths) && np >= (uint32_t)kSubWaves &&
                         cap >= 256u * kSubWaves) ? kSubWaves : 1;
       if (nsub > 1) {
         if (!ws->fork) {
