@@ -1,7 +1,8 @@
 """Autotuner for the BVH shape and the wavefront's launch shape.
 
 For a workload it times a small grid of the tunable knobs with CUDA events, keeps the fastest, and
-caches the choice in a JSON file keyed by the workload's shape and the GPU name:
+caches the choice in a JSON file keyed by the workload's shape and the GPU name (a choice timed on
+earlier kernels, or one that the grid does not hold, is searched again):
   - the tree (tune_build, tune_batch_build): children per wide node (BVH width 4 or 8; the node record keeps 8
     slots) and triangles per leaf, each candidate built and rendered;
   - the launch (tune_render, tune_batch): paths in flight (wave size), the idle-lane refill
@@ -27,6 +28,11 @@ import time
 import torch
 
 CACHE = os.environ.get("SWR_TUNE_CACHE", os.path.join(os.path.expanduser("~"), ".cache", "swr_b200", "tune.json"))
+
+# Counted up with every change of the kernels that may move a choice, or what a value of a knob means:
+# choices timed before it are searched again (trace_blocks 10, once the fastest, now only turns the
+# few-ray kernel off).
+KERNELS = 2
 
 BUILD_GRID = dict(width=[4, 8], max_leaf=[2, 3])
 RENDER_GRID = dict(wave_size=[1 << 22, 1 << 23, 1 << 24, 1 << 25, 1 << 26, 1 << 27], refill=[4, 8, 16], block_size=[128, 256, 512],
@@ -67,17 +73,23 @@ def _time(fn, reps):
     return best
 
 
+def _current(entry, grid):
+    """Whether a cached choice was timed on these kernels and is one of the grid's."""
+    return (entry is not None and entry.get("kernels") == KERNELS and set(entry["best"]) == set(grid) and
+            all(entry["best"][n] in grid[n] for n in grid))
+
+
 def _search(key, grid, run, reps, force):
     db = _load()
-    if key in db and not force:
-        return db[key]["best"]
     names = sorted(grid)
+    if not force and _current(db.get(key), grid):
+        return db[key]["best"]
     results = []
     for values in itertools.product(*[grid[n] for n in names]):
         cfg = dict(zip(names, values))
         results.append((_time(lambda: run(cfg), reps), cfg))
     results.sort(key=lambda r: r[0])
-    db[key] = {"best": results[0][1], "ms": results[0][0], "tried": [[ms, c] for ms, c in results],
+    db[key] = {"best": results[0][1], "ms": results[0][0], "kernels": KERNELS, "tried": [[ms, c] for ms, c in results],
                "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
     _store(db)
     return results[0][1]
