@@ -1404,6 +1404,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
   const unsigned trace_grid = (unsigned)(s->num_sms * std::max(trace_per_sm, 1));
   const unsigned shade_grid = shade_grid_for(s, cap, block);
 
+  unsigned bodies[kSubWaves] = {};  // rounds per iteration of each sub-wavefront's loop
   // Sub-wavefront h of a chunk: pixels [off, off + n) of it, queues of capw paths carved from the
   // h-th half of the queue buffer (the whole buffer when the chunk runs as one wavefront), control
   // block h; everything it launches goes to stream st. Graph path only.
@@ -1451,6 +1452,8 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     // rounds per iteration of the loop: what drains a chunk that is injected at once (its paths end
     // within max_depth rounds), when that is fewer than eight: an idle round takes about 5 us
     const unsigned body = (total <= capw && o->max_depth <= 8) ? (o->max_depth + 1u) & ~1u : 8u;
+    bodies[h] = body;
+    P.launches += want_samples ? 3 : 2;  // camera, resolve, dark samples
     std::vector<char> key(sizeof(DevScene) + sizeof(Frame) + sizeof(Qh) + 6 * sizeof(void*));
     {
       char* kp = key.data();
@@ -1496,7 +1499,8 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     return SWR_OK;
   };
   // what a drained sub-wavefront reports
-  auto collect = [&](const Ctrl& hc) -> int {
+  auto collect = [&](int h) -> int {
+    const Ctrl& hc = ws->host_ctrl[h];
     if (hc.status) return set_error(SWR_ERR_TIMEOUT, "swr: wavefront did not drain");
     P.rays += hc.rays;
     P.bounce_rays += hc.bounce_rays;
@@ -1504,7 +1508,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     P.node_visits += hc.nodes;
     P.tri_tests += hc.tris;
     P.iterations += hc.rounds;
-    P.launches += 2 + 2 * hc.rounds + hc.rounds / 8;  // camera, resolve, rounds, checks (at least)
+    P.launches += 2 * hc.rounds + hc.rounds / bodies[h];  // rounds, loop checks
     P.trace_launches += hc.rounds;
     return SWR_OK;
   };
@@ -1550,12 +1554,12 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
         for (int h = 1; h < nsub; ++h) SWR_CUDA(cudaStreamWaitEvent(stream, ws->join[h - 1], 0));
         SWR_CUDA(cudaStreamSynchronize(stream));
         for (int h = 0; h < nsub; ++h)
-          if ((rc = collect(ws->host_ctrl[h]))) return rc;
+          if ((rc = collect(h))) return rc;
       } else {
         if ((rc = launch_wave(0, stream, p0, 0, np, cap))) return rc;
         if ((rc = copy_out(stream, p0, 0, np))) return rc;
         SWR_CUDA(cudaStreamSynchronize(stream));
-        if ((rc = collect(ws->host_ctrl[0]))) return rc;
+        if ((rc = collect(0))) return rc;
       }
     } else {
       // profiled (or SWR_RENDER_HOST_LOOP): one wavefront whose loop the host runs, so that every
@@ -1576,7 +1580,7 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
       if ((rc = launch_camera(s, F, ws->ctrl, stream))) return rc;
       SWR_CUDA(timer.end(stream));
       SWR_CUDA(cudaGetLastError());
-      P.launches++;
+      P.launches += want_samples ? 2 : 1;
       Frame FR = F;
       FR.pixel0 = 0;
       FR.npix = 0;
