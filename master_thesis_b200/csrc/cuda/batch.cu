@@ -596,6 +596,7 @@ int ensure_bytes(void** p, size_t& have, size_t want) {
   cudaError_t e = cudaMalloc(p, std::max<size_t>(want, 256));
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // reported here, not by the next launch
     return set_error(SWR_ERR_ALLOC, "CUDA: batch workspace allocation of " + std::to_string(want) + " bytes failed");
   }
   have = want;

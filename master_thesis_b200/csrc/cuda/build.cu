@@ -575,6 +575,7 @@ int build_wide_bvh_device(const float* d_prim_boxes, uint32_t n, const DeviceBui
   SWR_CUDA(cudaMalloc(&words, ((size_t)n + 1) * 80));
   if (cudaMalloc(&order, (size_t)n * sizeof(uint32_t)) != cudaSuccess) {
     cudaFree(words);
+    cudaGetLastError();
     return set_error(SWR_ERR_ALLOC, "CUDA: BVH triangle order allocation failed");
   }
   out.d_nodes = words;

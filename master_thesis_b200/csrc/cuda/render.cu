@@ -1178,6 +1178,7 @@ int ensure(void** p, size_t& have, size_t want, size_t elem) {
   cudaError_t e = cudaMalloc(p, std::max<size_t>(want * elem, 256));
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // reported here, not by the next launch
     return set_error(SWR_ERR_ALLOC, std::string("CUDA: workspace allocation of ") +
                                         std::to_string(want * elem) + " bytes failed");
   }

@@ -14,6 +14,7 @@
 namespace swr {
 
 int cuda_fail(cudaError_t err, const char* what) {
+  cudaGetLastError();  // a call that failed (for lack of memory, say) is not the next launch's error
   return set_error(SWR_ERR_CUDA, std::string("CUDA: ") + what + ": " + cudaGetErrorString(err));
 }
 
@@ -34,6 +35,7 @@ int upload(void** dst, const std::vector<T>& v) {
   cudaError_t e = cudaMalloc(dst, bytes);
   if (e != cudaSuccess) {
     *dst = nullptr;
+    cudaGetLastError();
     return set_error(SWR_ERR_ALLOC, std::string("CUDA: cudaMalloc of ") + std::to_string(bytes) +
                                         " bytes failed: " + cudaGetErrorString(e));
   }
