@@ -100,7 +100,8 @@ struct Frame {
 
 // Sample index of a chunk -> pixel of the chunk, without a division: the host gives the multiplier
 // ceil(2^(31+l) / spp) with l = ceil(log2 spp), exact for indices below 2^31 (a chunk holds at most
-// 2^27 samples, or one pixel, whose quotient is 0: multiplier 0). Two 64-bit divisions per injected
+// 2^27 samples, the bidirectional tracer's fewer than 2^31, or either one pixel, whose quotient is 0:
+// multiplier 0). Two 64-bit divisions per injected
 // sample were a fifth of the shading kernel's instructions.
 constexpr uint32_t kDivOne = 0xFFu;
 __device__ __forceinline__ uint32_t div_spp(const Frame& F, uint32_t g) {
@@ -1801,6 +1802,10 @@ int render_bdpt_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts*
   const uint64_t chunk = o->wave_size ? (uint64_t)o->wave_size
                                       : std::max<uint64_t>(1u << 14, kBdptTableBytes / (48 * slots));
   const uint64_t px_per_chunk = std::max<uint64_t>(1, std::min<uint64_t>(npix_total, chunk / o->spp));
+  // (128 bytes a sample at least: more than the device holds, refused before the first of it is taken)
+  if (px_per_chunk > 1 && px_per_chunk * o->spp >= (1ull << 31))
+    return set_error(SWR_ERR_ALLOC, "swr: allocation of " + std::to_string(px_per_chunk * o->spp * (48 * slots + 32)) +
+                                        " bytes for a chunk of 2^31 samples or more");
   int rc;
   if ((rc = ensure(&ws->cam, ws->cam_bytes, px_per_chunk * 2 * sizeof(float4), 1))) return rc;
   if ((rc = ensure(&ws->contrib, ws->contrib_n, px_per_chunk * o->spp, sizeof(float4)))) return rc;

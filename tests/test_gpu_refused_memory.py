@@ -27,3 +27,17 @@ def test_next_call_after_a_refused_allocation(tmp_path):
     with pytest.raises(N.SwrError, match="allocation"):
         batch.render([big] * 16)
     assert torch.equal(batch.render([job])[0], image)
+
+
+def test_chunk_of_too_many_samples_takes_no_memory(tmp_path):
+    """2^32 samples at once: refused before any buffer of the chunk (68 GB of slots first) is taken."""
+    import torch
+    s = scenes.cornell(4, str(tmp_path))
+    sc = swr.Scene(swr.load_scene(s["scene"], s["basepath"]))
+    cam = swr.load_camera(s["camera"], 1024, 1024)
+    out = torch.empty((1024, 1024, 3), device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    with pytest.raises(N.SwrError, match="allocation"):
+        sc.render_bdpt(cam, 1024, 1024, 4096, 5, 5, 5, chunk=0xFFFFFFFF, out=out)
+    assert free - torch.cuda.mem_get_info()[0] < 1 << 30
