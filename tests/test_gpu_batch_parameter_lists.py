@@ -57,3 +57,38 @@ def test_lists_of_different_lengths():
     assert len(a) == len(b) == 2 and all(torch.equal(x, y) for x, y in zip(a, b))
     with pytest.raises((ValueError, IndexError)):
         diff.render_physical_batch(batch, jobs, alb[:1], em[:1])
+
+
+def test_table_is_not_overwritten_while_its_launch_waits():
+    """The first call's launch waits for room on a GPU that closest-hit queries fill, its table already
+    copied; the second call, on another stream, must not copy its own over it. All scenes are of one size,
+    so that whichever table a launch reads fits them."""
+    import torch
+    datas = [scenes.random_scene(60 + k, 256)[0] for k in range(2)]
+    alb = [torch.rand((d.num_triangles, 3), generator=torch.Generator().manual_seed(k)).cuda()
+           for k, d in enumerate(datas)]
+    em = [torch.full((d.num_objects, 3), 2.0 + k, device="cuda") for k, d in enumerate(datas)]
+    assert alb[0].shape == alb[1].shape and em[0].shape == em[1].shape
+    one, many = [swr.Scene(d) for d in datas], [swr.Scene(d) for d in datas]
+    busy = swr.Scene(scenes.random_scene(9, 100_000)[0])
+    o, d = scenes.uniform_rays(1 << 22, busy.data.vpos.min(0), busy.data.vpos.max(0), 5)
+    hits = torch.empty((1 << 22, 4), dtype=torch.int32, device="cuda")
+    batch = swr.Batch()
+    batch.set_parameters(many, alb[::-1], em[::-1])  # the buffers exist before the queries run
+    filler, a, b = (torch.cuda.Stream() for _ in range(3))
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    for _ in range(8):
+        busy.trace(o, d, out=hits, stream=filler)
+    done.record(filler)
+    batch.set_parameters([many[0]], [alb[0]], [em[0]], stream=a)
+    batch.set_parameters([many[1]], [alb[1]], [em[1]], stream=b)
+    queued_behind_the_queries = not done.query()
+    torch.cuda.synchronize()
+    assert queued_behind_the_queries
+    cam = swr.make_camera((4.0, 2.5, 4.0), (-0.75, -0.3), W, H, fov_deg=60.0)
+    for k in range(2):
+        one[k].set_albedo(alb[k])
+        one[k].set_emission(em[k])
+        x = _image(one[k], cam)
+        assert int(torch.count_nonzero(x)) > 0 and torch.equal(x, _image(many[k], cam))
