@@ -292,8 +292,10 @@ typedef struct swr_bdpt_opts {
   uint32_t shade_batch;  /* lanes of a warp with a finished trace that advance together, bits 0-7
                             for the path stages and bits 8-15 for the connection queries (each
                             1..32, 0 = the library's choice) */
-  uint32_t blocks_per_sm;  /* resident blocks per SM targeted by the register budget: 0 (compiler's
-                              choice), 5, 6 or 8 */
+  uint32_t blocks_per_sm;  /* resident blocks per SM targeted by the register budgets of both kernels,
+                              5, 6 or 8; 0: the library's choice (5 for the paths, the compiler's for
+                              the connections, and kernels of their own for scenes of at most 2,048
+                              triangles, which the other values do not take) */
 } swr_bdpt_opts;
 int swr_render_bdpt(swr_scene* scene, const swr_camera* cam, const swr_render_opts* opts,
                     const swr_bdpt_opts* bdpt, float* rgb_out, float* samples_out, void* stream);

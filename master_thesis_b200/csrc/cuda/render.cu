@@ -2,19 +2,20 @@
 //
 // Work decomposition: a global sample index g = pixel * spp + sample over the image (processed
 // in pixel chunks). Per chunk:
-//   k_camera   one thread per pixel: primary ray through the pixel centre and the reference's
+//   k_camera   one lane per pixel (eight in chunks of few pixels): primary ray through the pixel centre and the reference's
 //              back-face skipping prefix (path_tracer.cpp:50-57). This prefix uses no random
 //              numbers, so it is the same for every sample of the pixel and is traced once per
 //              pixel; its first scattering hit is stored in a per-pixel record.
 //   loop until no path is live and every sample has been injected:
 //     k_shade  shades the traced queue and injects new samples (taking their first hit from the
 //              pixel record) up to the queue capacity; continuing paths are appended to the other
-//              queue with one atomic per warp (ballot + popc compaction); finished samples write
-//              their radiance to a per-sample slot.
+//              queue with one atomic per warp (ballot + popc compaction); samples that reach a
+//              light write their radiance to a per-sample slot and set their bit.
 //     k_trace  persistent closest-hit traversal over the new queue.
-//   k_resolve  sums each pixel's sample slots in sample order and scales, as renderPixel does.
+//   k_resolve  sums each pixel's lit slots in sample order and scales, as renderPixel does.
 // Queue counters and the injection window live in a small device control block that the
-// kernels advance themselves, so the host only launches kernels and polls completion.
+// kernels advance themselves, so the host only launches a graph whose loop ends on the device
+// (or, profiled or asked to, the rounds themselves) and waits once per chunk.
 #include <algorithm>
 #include <cstring>
 #include <mutex>

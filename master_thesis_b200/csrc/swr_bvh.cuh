@@ -175,16 +175,7 @@ SWR_HD float4 ldg4(const float4* p) {
 #endif
 }
 
-// max / min of three floats, NaN operands ignored as by fmaxf / fminf
-SWR_HD float fmax3(float a, float b, float c) {
-#if defined(__CUDA_ARCH__)
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-#else
-  return fmaxf(fmaxf(a, b), c);
-#endif
-}
+// min of three floats, NaN operands ignored as by fminf
 SWR_HD float fmin3(float a, float b, float c) {
 #if defined(__CUDA_ARCH__)
   float r;
@@ -285,7 +276,8 @@ struct Traversal {
     st.bind(mem);
     prepare(mem);
   }
-  // mem: the block's kTraceRows rows (a kernel's own array, so that its address is a constant)
+  // mem: the block's kTraceMem rows (a kernel's own 1024-byte aligned array, so that its address is a
+  // constant), of which prepare() has filled the last two
   SWR_HD void init(f3 o_, f3 d_, uint2* mem) {
     o = o_;
     d = d_;
@@ -544,8 +536,8 @@ struct Traversal {
 };
 
 // Closest hit of ray (o, d), run to completion. obj_boxes/tri_boxes hold the reference's own
-// boxes (lo.xyz, hi.xyz) per object and per triangle record; mem: the block's kTraceRows rows (host
-// build: kStackShared entries). Returns false on a miss.
+// boxes (lo.xyz, hi.xyz) per object and per triangle record; mem: the block's kTraceMem rows, after
+// Traversal::prepare (host build: kStackShared entries); the int is not used. Returns false on a miss.
 template <bool kStats, bool kPostpone = false, int kRule = kRuleReference>
 SWR_HD bool trace_closest(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                           const float* __restrict__ tri_boxes, const float* __restrict__ obj_boxes,
