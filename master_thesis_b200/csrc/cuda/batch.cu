@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ct
           depth = J.depth;
           const uint32_t pix = (uint32_t)(p - J.pixel_base);
           d = swrx::primary_dir(J.vi, J.pi, pix % J.W, pix / J.W, J.W, J.H);
-          tr.init(mk(J.org[0], J.org[1], J.org[2]), d, stack);
+          tr.init(mk(J.org[0], J.org[1], J.org[2]), d, stack, sc->ray_flags);
           ++traced;
           active = true;
         }
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ct
         const f3 n = swrx::shading_normal(sc->tris, sc->shade, tr.hit_slot(stack), hp);
         if (swrx::vdot(n, d) > 0.0f) {
           if (i + 1 < depth) {
-            tr.init(swrx::vadd(hp, swrx::vscale(0.01f, d)), d, stack);
+            tr.init(swrx::vadd(hp, swrx::vscale(0.01f, d)), d, stack, sc->ray_flags);
             ++i;
             ++traced;
             done = false;
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kTB) k_btrace_wide(BArgs A, BCtrl* __restrict_
     const float4 o = q.o[i], d = q.d[i];
     const DevScene& sc = A.scenes[A.jobs[__float_as_uint(q.c[i].w) >> 16].scene];
     const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
-        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr);
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr, sc.ray_flags);
     if ((lane() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
   }
 }
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ 
             const float4 o = q.o[j], d = q.d[j];
             const uint32_t job = __float_as_uint(q.c[j].w) >> 16;
             sc = &A.scenes[A.jobs[job].scene];
-            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack);
+            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, sc->ray_flags);
             tr.st.set(stack, swrx::kRowUser, make_uint2(j, 0u));
             active = true;
           }
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kTB, 9) k_badjoint(BArgs A, BCtrl* __restrict_
         swrx::shade_physical_adj(sc->tris, sc->shade, sc->mats, sc->albedo, pend_slot, pend_t, P, st, av);
     if (outcome == swrx::kContinue) {
       tape.push(pend_slot, c_before, av);
-      tr.init(st.o, st.d, stack);
+      tr.init(st.o, st.d, stack, sc->ray_flags);
       tracing = true;
       continue;
     }

@@ -14,6 +14,7 @@
 //   k_inst_derive    one thread per triangle: edges, dot products, reference triangle box and
 //                    corner normals, written to the triangle's BVH slot; the scene extent is
 //                    reduced for the traversal boxes' margin.
+//   k_inst_area      (only for scenes with coordinates from 2,048 on) the share of flat boxes.
 //   k_inst_prims     traversal boxes (reference boxes widened by the margin of scene_pack.cpp).
 //   k_refit          one launch per tree level, deepest first: each wide node's child boxes from
 //                    its children's exact boxes or its leaves' traversal boxes, requantised on a
@@ -29,6 +30,7 @@
 #include <vector>
 
 #include "../host/capi_common.h"
+#include "../host/scene_pack.h"
 #include "../plane_grid.h"
 #include "swr_internal.cuh"
 
@@ -50,6 +52,7 @@ struct InstView {
   float* node_box;              // [6 * nodes] exact union boxes
   uint32_t* order;              // nodes by level, deepest level first
   unsigned* ext;                // [6] ordered-int scene extent
+  double* area;                 // [2] of all triangles, and of those with a flat box (k_inst_area)
   unsigned* bad;                // [1] set when a world vertex or normal comes out non-finite
   uint32_t nv, nt, no, nlt;
 };
@@ -274,6 +277,29 @@ __global__ void k_inst_rank(InstView I, DevScene sc, float4* __restrict__ tris) 
   reinterpret_cast<uint32_t*>(tris + 3 * (size_t)s + 2)[2] = I.base[I.tri_obj[t]] + I.local_rank[t];
 }
 
+// areas of all triangles and of those whose reference box is flat (as scene_pack.cpp's flat_share)
+__global__ void k_inst_area(InstView I, const float4* __restrict__ tris, const float* __restrict__ tri_boxes,
+                            uint32_t ns) {
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  double all = 0.0, flat = 0.0;
+  if (s < ns) {
+    const float4 a = tris[3 * (size_t)s], b = tris[3 * (size_t)s + 1], c = tris[3 * (size_t)s + 2];
+    const double x0 = a.w, y0 = b.x, z0 = b.y, x1 = b.z, y1 = b.w, z1 = c.x;
+    const double nx = y0 * z1 - z0 * y1, ny = z0 * x1 - x0 * z1, nz = x0 * y1 - y0 * x1;
+    all = sqrt(nx * nx + ny * ny + nz * nz);
+    const float* box = tri_boxes + 6 * (size_t)s;
+    if (!(box[0] < box[3] && box[1] < box[4] && box[2] < box[5])) flat = all;
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    all += __shfl_xor_sync(0xffffffffu, all, off);
+    flat += __shfl_xor_sync(0xffffffffu, flat, off);
+  }
+  if ((threadIdx.x & 31u) == 0) {
+    atomicAdd(&I.area[0], all);
+    atomicAdd(&I.area[1], flat);
+  }
+}
+
 // traversal boxes: the reference triangle boxes widened by the margin scene_pack.cpp uses
 __global__ void k_inst_prims(InstView I, const float* __restrict__ tri_boxes, uint32_t ns) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -439,6 +465,7 @@ int attach(swr_scene* s, const swr_host_scene* hs, const swr_scene_desc& d) {
   if ((rc = I->alloc(&I->v.node_box, 6 * (size_t)s->dev.num_nodes))) return rc;
   if ((rc = I->alloc(&I->v.ext, 6))) return rc;
   if ((rc = I->alloc(&I->v.bad, 1))) return rc;
+  if ((rc = I->alloc(&I->v.area, 2))) return rc;
   if (cudaMallocHost(&I->host_boxes, sizeof(float) * (6 * std::max<size_t>(I->v.no, 1) + 1)) != cudaSuccess) {
     cudaGetLastError();
     I->host_boxes = nullptr;
@@ -562,8 +589,20 @@ int swr_scene_set_transforms(swr_scene* s, const swr_object_transform* xf, uint3
   SWR_CUDA(cudaMemcpyAsync(I->v.base, base.data(), base.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
   swr::k_inst_rank<<<swr::blocks(I->v.nt, 256), 256, 0, stream>>>(I->v, s->dev, (float4*)s->d_tris);
   SWR_CUDA(cudaGetLastError());
+  // boxes can only be flat from kFlatFrom on
+  double area[2] = {0.0, 0.0};
+  float mabs = 0.0f;
+  for (size_t i = 0; i < 6 * (size_t)n; ++i) mabs = std::max(mabs, std::fabs(boxes[i]));
+  if (mabs >= swr::kFlatFrom) {
+    SWR_CUDA(cudaMemsetAsync(I->v.area, 0, sizeof(area), stream));
+    swr::k_inst_area<<<swr::blocks(s->dev.num_slots, 256), 256, 0, stream>>>(
+        I->v, (const float4*)s->d_tris, (const float*)s->d_tri_boxes, s->dev.num_slots);
+    SWR_CUDA(cudaGetLastError());
+    SWR_CUDA(cudaMemcpyAsync(area, I->v.area, sizeof(area), cudaMemcpyDeviceToHost, stream));
+  }
   std::copy(xf, xf + n, I->xf.begin());
   SWR_CUDA(cudaStreamSynchronize(stream));  // the host arrays above go out of scope
+  s->dev.ray_flags = swr::first_ray_flags(area[0] > 0.0 ? area[1] / area[0] : 0.0);
   return SWR_OK;
 }
 

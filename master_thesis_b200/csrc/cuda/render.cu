@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
           i = 0;
           const uint32_t pix = F.pixel0 + k;
           d = swrx::primary_dir(F.vi, F.pi, pix % F.W, pix / F.W, F.W, F.H);
-          tr.init(org, d, stack);
+          tr.init(org, d, stack, sc.ray_flags);
           ++traced;
           active = true;
         }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
         const f3 n = swrx::shading_normal(sc.tris, sc.shade, tr.hit_slot(stack), p);
         if (swrx::vdot(n, d) > 0.0f) {
           if (i + 1 < F.depth) {
-            tr.init(swrx::vadd(p, swrx::vscale(0.01f, d)), d, stack);
+            tr.init(swrx::vadd(p, swrx::vscale(0.01f, d)), d, stack, sc.ray_flags);
             ++i;
             ++traced;
             done = false;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera_wide(DevScene sc, Frame 
     float4 rec0 = make_float4(0, 0, 0, 0), rec1 = make_float4(0, 0, 0, __uint_as_float(kDeadSlot));
     for (uint32_t i = 0; i < F.depth; ++i) {
       const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
-          sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, o, d, stack, nullptr);
+          sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, o, d, stack, nullptr, sc.ray_flags);
       traced += first;
       if (h.slot == kDeadSlot) break;
       const f3 p = swrx::hit_point(o, d, h.t);
@@ -469,7 +469,8 @@ __global__ void __launch_bounds__(kTraceBlock)
   for (unsigned i = swrx::wide_first(); i < n; i += swrx::wide_stride()) {
     const float4 o = q.o[i], d = q.d[i];
     const swrx::WideHit h = swrx::wide_closest<kStats, swrx::kRuleReference>(
-        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, &st);
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, &st,
+        sc.ray_flags);
     if ((lane_id() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
   }
   if (kStats) add_stats(ctrl, st);
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(kTraceBlock)
       const float4 o = q.o[i], d = q.d[i];
       swrx::Hit h;
       swrx::trace_closest<kStats>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z),
-                                  mk(d.x, d.y, d.z), stack, kTraceBlock, h, &st);
+                                  mk(d.x, d.y, d.z), stack, kTraceBlock, h, &st, sc.ray_flags);
       q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
     }
   }
@@ -542,7 +543,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
           const unsigned j = base + __popc(idle & lt);
           if (j < n) {
             const float4 o = __ldcs(q.o + j), d = __ldcs(q.d + j);
-            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack);
+            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, sc.ray_flags);
             tr.st.set(stack, swrx::kRowUser, make_uint2(j, 0u));
             active = true;
           }
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(kTraceBlock)
     // emitter (depth reached, Russian roulette, escape) carries no radiance and no gradient
     if (outcome == swrx::kContinue) {
       tape.push(pend_slot, c_before, av);
-      tr.init(st.o, st.d, stack);
+      tr.init(st.o, st.d, stack, sc.ray_flags);
       tracing = true;
       continue;
     }
@@ -846,7 +847,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
           }
           continue;
         }
-        tr.init(o, d, stack);
+        tr.init(o, d, stack, sc.ray_flags);
         tracing = true;
       } else if (phase == kVisionDone) {
         if (vlight) {  // c is the throughput recorded at the last vision vertex
@@ -885,7 +886,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
         i = 1;
         if (B.lj > 1) {
           phase = kLight;
-          tr.init(o, d, stack);
+          tr.init(o, d, stack, sc.ray_flags);
           tracing = true;
         } else {
           B.head[q] = make_uint4(vfirst, dv, dl, 0u);
@@ -988,7 +989,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
       const f3 dd = swrx::vsub(b, a);
       const float dist2 = swrx::vdot(dd, dd);
       dn = swrx::vnormalize(dd);
-      tr.init_occlusion(a, dn, dist2, stack);
+      tr.init_occlusion(a, dn, dist2, stack, sc.ray_flags);
       tracing = true;
       pending = true;
       break;

@@ -27,6 +27,7 @@ struct DevScene {
   const uint4* lights;      // [num_lights]      first light triangle, count, object, 0
   const float4* light_tris; // [5 per triangle]  corners v0 v1 v2 and corner normals n0 n1 n2
   uint32_t num_nodes, num_slots, num_objects, num_tris, num_lights;
+  uint32_t ray_flags;       // flags that rays start with (first_ray_flags)
 };
 
 }  // namespace swr
@@ -67,6 +68,9 @@ int cuda_fail(cudaError_t err, const char* what);
     cudaError_t _e = (call);                             \
     if (_e != cudaSuccess) return swr::cuda_fail(_e, #call); \
   } while (0)
+
+// DevScene::ray_flags by the share of the triangles' area whose reference boxes are flat
+uint32_t first_ray_flags(double flat_share);
 
 // true when p is host memory that the device cannot address directly
 bool is_host_pointer(const void* p);

@@ -20,6 +20,21 @@ static inline float ubits(uint32_t u) {
   return f;
 }
 
+// Share of the triangles' area that lies in triangles whose reference box is flat.
+static double flat_share(const PackedScene& s) {
+  double area = 0.0, flat = 0.0;
+  for (size_t k = 0; k < s.slot_to_id.size(); ++k) {
+    const float4 a = s.tris[3 * k], b = s.tris[3 * k + 1], c = s.tris[3 * k + 2];
+    const double e0[3] = {a.w, b.x, b.y}, e1[3] = {b.z, b.w, c.x};
+    const double n[3] = {e0[1] * e1[2] - e0[2] * e1[1], e0[2] * e1[0] - e0[0] * e1[2], e0[0] * e1[1] - e0[1] * e1[0]};
+    const double x = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    const float *lo = &s.tri_boxes[6 * k], *hi = lo + 3;
+    area += x;
+    if (!(lo[0] < hi[0] && lo[1] < hi[1] && lo[2] < hi[2])) flat += x;
+  }
+  return area > 0.0 ? flat / area : 0.0;
+}
+
 int pack_scene(const swr_scene_desc* d, const swr_build_opts* opts, PackedScene& out, bool host_bvh) {
   int rc = validate_desc(d);
   if (rc) return rc;
@@ -118,6 +133,7 @@ int pack_scene(const swr_scene_desc* d, const swr_build_opts* opts, PackedScene&
       }
     }
   });
+  if (mabs >= kFlatFrom) out.flat_share = flat_share(out);
   {
     // triangles of each object are contiguous in id order (tri_object is non-decreasing)
     std::vector<uint32_t> first(no + 1, 0);

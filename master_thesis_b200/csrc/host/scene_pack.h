@@ -11,6 +11,10 @@
 
 namespace swr {
 
+// The reference widens a triangle's box by 1e-4 each way; from this coordinate on, where floats are more
+// than 2e-4 apart, the rounding can take that back and leave a box without extent on an axis.
+constexpr float kFlatFrom = 2048.0f;
+
 struct PackedScene {
   std::vector<uint32_t> nodes;    // 20 words per wide node
   std::vector<float4> tris;       // 3 per slot: v0|e0|e1|id rank obj
@@ -28,6 +32,7 @@ struct PackedScene {
   std::vector<uint32_t> lights;
   std::vector<float4> light_tris;
   uint32_t num_nodes = 0, depth = 0;
+  double flat_share = 0.0;  // of the triangles' area, in triangles whose box has no extent on an axis
 };
 
 // Validates and packs; returns SWR_OK or an error code (message in swr_last_error). With

@@ -31,7 +31,8 @@
 // is kept without the slab tests. Only the finished ray's hit is put to both reference slab tests
 // (Traversal::settled): when it passes, it is the best of all candidates and a valid one, so it is
 // the best valid one; when it fails (a hit on the very rim of its triangle's box), the ray is
-// traced once more with the tests made on every candidate. The kernels settle the finished rays of
+// traced once more with the tests made on every candidate (in scenes where whole walls fail, they are
+// made on every candidate from the start: DevScene::ray_flags). The kernels settle the finished rays of
 // a warp together, at the next refill: the tests are a third of a step's instructions, and made at
 // each acceptance they ran for one or two lanes in nearly every step of a warp.
 #pragma once
@@ -278,7 +279,8 @@ struct Traversal {
   }
   // mem: the block's kTraceMem rows (a kernel's own 1024-byte aligned array, so that its address is a
   // constant), of which prepare() has filled the last two
-  SWR_HD void init(f3 o_, f3 d_, uint2* mem) {
+  // flags: 0, or kStrict for the slab tests on every candidate from the start (DevScene::ray_flags)
+  SWR_HD void init(f3 o_, f3 d_, uint2* mem, uint32_t flags = 0u) {
     o = o_;
     d = d_;
     host_turn = f2bits(o_.x) ^ f2bits(d_.y);
@@ -291,7 +293,7 @@ struct Traversal {
     idz = 1.0f / dz;
     oct = (idx < 0.0f ? 1u : 0u) | (idy < 0.0f ? 2u : 0u) | (idz < 0.0f ? 4u : 0u);
     st.bind(mem);
-    start(mem, 0u, INFINITY);
+    start(mem, flags, INFINITY);
   }
 
   // the ray at the root, with no hit yet
@@ -309,9 +311,9 @@ struct Traversal {
   // rule is the closest-hit one started from a best of (dist2, no rank), whose first acceptance is
   // exactly "d2 <= dist2"; nodes beyond sqrt(dist2) (with the pruning slack) are skipped, which
   // keeps every such candidate because d is of unit length.
-  SWR_HD void init_occlusion(f3 o_, f3 d_, float dist2, uint2* mem) {
+  SWR_HD void init_occlusion(f3 o_, f3 d_, float dist2, uint2* mem, uint32_t flags = 0u) {
     init(o_, d_, mem);
-    start(mem, kAny, dist2);
+    start(mem, kAny | flags, dist2);
     tprune = sqrtf(dist2) * kPruneSlack;
   }
 
@@ -541,9 +543,9 @@ struct Traversal {
 template <bool kStats, bool kPostpone = false, int kRule = kRuleReference>
 SWR_HD bool trace_closest(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                           const float* __restrict__ tri_boxes, const float* __restrict__ obj_boxes,
-                          f3 o, f3 d, uint2* mem, int, Hit& hit, TraceStats* stats) {
+                          f3 o, f3 d, uint2* mem, int, Hit& hit, TraceStats* stats, uint32_t flags = 0u) {
   Traversal tr;
-  tr.init(o, d, mem);
+  tr.init(o, d, mem, flags);
   for (;;) {
     while (!tr.template step<kStats, kPostpone, kRule>(nodes, tris, tri_boxes, obj_boxes, mem, stats)) {
     }

@@ -33,11 +33,11 @@ struct WideHit {
 };
 
 // The calling lane's group works on one ray (o, d), the same in its eight lanes; mem: the block's
-// rows, of which the group uses its own kStackTotal entries.
+// rows, of which the group uses its own kStackTotal entries; flags: as Traversal::init.
 template <bool kStats, int kRule>
 __device__ __forceinline__ WideHit wide_closest(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                                              const float* __restrict__ tri_boxes, const float* __restrict__ obj_boxes,
-                                             f3 o, f3 d, uint2* mem, TraceStats* stats) {
+                                             f3 o, f3 d, uint2* mem, TraceStats* stats, uint32_t flags) {
   const uint32_t c = threadIdx.x & 7u, shift = threadIdx.x & 24u;
   const uint32_t gmask = 0xFFu << shift;
   uint2* stack = mem + (threadIdx.x / kWideLanes) * kStackTotal;
@@ -50,7 +50,7 @@ __device__ __forceinline__ WideHit wide_closest(const float4* __restrict__ nodes
   const uint32_t nx = 32u + c + ((oct & 1u) ? 24u : 0u), fx = 32u + c + ((oct & 1u) ? 0u : 24u);
   const uint32_t ny = 40u + c + ((oct & 2u) ? 24u : 0u), fy = 40u + c + ((oct & 2u) ? 0u : 24u);
   const uint32_t nz = 48u + c + ((oct & 4u) ? 24u : 0u), fz = 48u + c + ((oct & 4u) ? 0u : 24u);
-  for (bool strict = false;; strict = true) {
+  for (bool strict = flags & Traversal::kStrict;; strict = true) {
     uint32_t bslot = 0xFFFFFFFFu, bkey = 0xFFFFFFFFu;
     float bt = INFINITY, bd2 = INFINITY, tprune = INFINITY;
     uint2 ng = make_uint2(0u, (1u << (24 + oct)) | 1u);
