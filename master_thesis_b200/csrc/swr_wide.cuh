@@ -50,7 +50,7 @@ __device__ __forceinline__ WideHit wide_closest(const float4* __restrict__ nodes
   const uint32_t nx = 32u + c + ((oct & 1u) ? 24u : 0u), fx = 32u + c + ((oct & 1u) ? 0u : 24u);
   const uint32_t ny = 40u + c + ((oct & 2u) ? 24u : 0u), fy = 40u + c + ((oct & 2u) ? 0u : 24u);
   const uint32_t nz = 48u + c + ((oct & 4u) ? 24u : 0u), fz = 48u + c + ((oct & 4u) ? 0u : 24u);
-  for (bool strict = flags & Traversal::kStrict;; strict = true) {
+  for (bool strict = kRule == kRuleReference && (flags & Traversal::kStrict);; strict = true) {
     uint32_t bslot = 0xFFFFFFFFu, bkey = 0xFFFFFFFFu;
     float bt = INFINITY, bd2 = INFINITY, tprune = INFINITY;
     uint2 ng = make_uint2(0u, (1u << (24 + oct)) | 1u);

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import master_thesis_b200 as swr
-from master_thesis_b200 import scenes
+from master_thesis_b200 import rt, scenes
 from master_thesis_b200.api import MAT_DTYPE
 from oracle import oracle as O
 
@@ -74,6 +74,24 @@ def test_hits_and_images(at, big, builder):
     got = sc.render_bdpt(c2, w, h, 4, 4, 3, 5, seed=5).cpu().numpy().reshape(-1, 3)
     _, bd = O.render_bdpt(osc, O.camera(*swr.camera_arrays(c2)), w, h, 4, 4, 3, 5, 5)
     assert np.allclose(got, bd, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("at", [0.0, 2050.0, 8192.0])
+@pytest.mark.parametrize("n", [3000, 30000])
+def test_ray_queries_know_no_boxes(at, n):
+    """The ray tracing pipeline's closest hit has no slab test: the flat wall is there at any distance."""
+    import torch
+    sd = _scene(at, False)
+    rng = np.random.default_rng(4)
+    o, d = np.zeros((n, 4), np.float32), np.zeros((n, 4), np.float32)
+    o[:, :3] = rng.uniform((at - 2, -4, -4), (at + 6, 4, 4), (n, 3))
+    v = rng.normal(size=(n, 3)) * (1.0, 0.3, 0.3)
+    d[:, :3] = v / np.linalg.norm(v, axis=1, keepdims=True)
+    tri, t = O.rt_trace(O.OracleScene.from_scene_data(sd), o, d)
+    assert np.mean(sd.tri_obj[np.minimum(tri, 5)][tri != 0xFFFFFFFF] == 1) > 0.2
+    got = rt.trace(swr.Scene(sd), torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()).cpu().numpy().view(np.uint32)
+    hit = tri != 0xFFFFFFFF
+    assert np.array_equal(got[:, 0], tri) and np.array_equal(got[hit, 3], t[hit].view(np.uint32))
 
 
 def _visits(sc, o, d):
