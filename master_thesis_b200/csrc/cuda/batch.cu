@@ -79,6 +79,7 @@ struct BArgs {
   uint64_t npix;  // total pixels
   uint32_t capacity, refill;
   uint32_t batch;               // adjoint: lanes with a finished trace that shade together
+  uint32_t ray_flags;           // flags that rays start with (first_ray_flags)
   float4* cam;                  // [npix*2]
   unsigned long long* accum;    // [npix*3] fixed point
 };
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ct
           depth = J.depth;
           const uint32_t pix = (uint32_t)(p - J.pixel_base);
           d = swrx::primary_dir(J.vi, J.pi, pix % J.W, pix / J.W, J.W, J.H);
-          tr.init(mk(J.org[0], J.org[1], J.org[2]), d, stack, sc->ray_flags);
+          tr.init(mk(J.org[0], J.org[1], J.org[2]), d, stack, A.ray_flags);
           ++traced;
           active = true;
         }
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kTB) k_bcamera(BArgs A, BCtrl* __restrict__ ct
         const f3 n = swrx::shading_normal(sc->tris, sc->shade, tr.hit_slot(stack), hp);
         if (swrx::vdot(n, d) > 0.0f) {
           if (i + 1 < depth) {
-            tr.init(swrx::vadd(hp, swrx::vscale(0.01f, d)), d, stack, sc->ray_flags);
+            tr.init(swrx::vadd(hp, swrx::vscale(0.01f, d)), d, stack, A.ray_flags);
             ++i;
             ++traced;
             done = false;
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(kTB) k_btrace_wide(BArgs A, BCtrl* __restrict_
     const float4 o = q.o[i], d = q.d[i];
     const DevScene& sc = A.scenes[A.jobs[__float_as_uint(q.c[i].w) >> 16].scene];
     const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
-        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr, sc.ray_flags);
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr, A.ray_flags);
     if ((lane() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
   }
 }
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(kTB, 9) k_btrace(BArgs A, BCtrl* __restrict__ 
             const float4 o = q.o[j], d = q.d[j];
             const uint32_t job = __float_as_uint(q.c[j].w) >> 16;
             sc = &A.scenes[A.jobs[job].scene];
-            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, sc->ray_flags);
+            tr.init(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, A.ray_flags);
             tr.st.set(stack, swrx::kRowUser, make_uint2(j, 0u));
             active = true;
           }
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(kTB, 9) k_badjoint(BArgs A, BCtrl* __restrict_
         swrx::shade_physical_adj(sc->tris, sc->shade, sc->mats, sc->albedo, pend_slot, pend_t, P, st, av);
     if (outcome == swrx::kContinue) {
       tape.push(pend_slot, c_before, av);
-      tr.init(st.o, st.d, stack, sc->ray_flags);
+      tr.init(st.o, st.d, stack, A.ray_flags);
       tracing = true;
       continue;
     }
@@ -627,7 +628,8 @@ namespace {
 // Appends one job to the table (validating what the primal and the adjoint both need); uniq / hs
 // collect the distinct scenes, samples / pixels the running prefix sums.
 int add_job(int device, const swr_scene* scene, const swr_camera& cam, const swr_render_opts& o, BJob& d,
-            std::vector<const swr_scene*>& uniq, std::vector<DevScene>& hs, uint64_t& samples, uint64_t& pixels) {
+            std::vector<const swr_scene*>& uniq, std::vector<DevScene>& hs, uint64_t& samples, uint64_t& pixels,
+            double& flat) {
   if (!scene) return set_error(SWR_ERR_INVALID, "swr: batch job without scene");
   if (scene->device != device) return set_error(SWR_ERR_INVALID, "swr: batch jobs on another device");
   if (o.width == 0 || o.height == 0 || o.spp == 0) return set_error(SWR_ERR_INVALID, "swr: zero image size");
@@ -662,6 +664,7 @@ int add_job(int device, const swr_scene* scene, const swr_camera& cam, const swr
   const uint64_t np = (uint64_t)o.width * o.height;
   pixels += np;
   samples += np * o.spp;
+  flat += (double)(np * o.spp) * scene->flat_share;
   return SWR_OK;
 }
 
@@ -717,12 +720,13 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   std::vector<DevScene> hs;
   std::vector<const swr_scene*> uniq;
   uint64_t samples = 0, pixels = 0;
+  double flat = 0.0;  // samples times their scene's share of flat boxes
   int num_sms = 0;
   int rc;
   for (uint32_t k = 0; k < n; ++k) {
     const swr_batch_job& J = jobs[k];
     if (!J.rgb_out) return set_error(SWR_ERR_INVALID, "swr: batch job without output");
-    if ((rc = add_job(b->device, J.scene, J.cam, J.opts, hj[k], uniq, hs, samples, pixels))) return rc;
+    if ((rc = add_job(b->device, J.scene, J.cam, J.opts, hj[k], uniq, hs, samples, pixels, flat))) return rc;
     if (is_host_pointer(J.rgb_out)) return set_error(SWR_ERR_INVALID, "swr: batch outputs must be device memory");
     hj[k].out = J.rgb_out;
     num_sms = J.scene->num_sms;
@@ -750,6 +754,7 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   A.npix = pixels;
   A.capacity = cap;
   A.refill = refill;
+  A.ray_flags = first_ray_flags(flat / (double)samples);
   A.cam = (float4*)b->cam;
   A.accum = (unsigned long long*)b->accum;
   uint32_t maxdepth = 0;
@@ -967,6 +972,7 @@ int swr_render_adjoint_batch(swr_batch* b, const swr_adjoint_job* jobs, uint32_t
   std::vector<DevScene> hs;
   std::vector<const swr_scene*> uniq;
   uint64_t samples = 0, pixels = 0;
+  double flat = 0.0;  // samples times their scene's share of flat boxes
   int num_sms = 0;
   int rc;
   // distinct gradient buffers and their sizes in bytes (zeroed once each; jobs that share a
@@ -989,7 +995,7 @@ int swr_render_adjoint_batch(swr_batch* b, const swr_adjoint_job* jobs, uint32_t
       return set_error(SWR_ERR_INVALID, "swr: the adjoint is defined for SWR_MODE_PHYSICAL");
     if (J.opts.max_depth > (uint32_t)swrx::kAdjMaxDepth)
       return set_error(SWR_ERR_UNSUPPORTED, "swr: the adjoint supports max_depth 1..16");
-    if ((rc = add_job(b->device, J.scene, J.cam, J.opts, hj[k], uniq, hs, samples, pixels))) return rc;
+    if ((rc = add_job(b->device, J.scene, J.cam, J.opts, hj[k], uniq, hs, samples, pixels, flat))) return rc;
     if (is_host_pointer(J.dl_dimage) || is_host_pointer(J.dl_dalbedo) || is_host_pointer(J.dl_demission))
       return set_error(SWR_ERR_INVALID, "swr: the adjoint takes device buffers");
     hj[k].dl = J.dl_dimage;
@@ -1028,6 +1034,7 @@ int swr_render_adjoint_batch(swr_batch* b, const swr_adjoint_job* jobs, uint32_t
   A.npix = pixels;
   A.refill = refill;
   A.batch = batch;
+  A.ray_flags = first_ray_flags(flat / (double)samples);
   A.cam = (float4*)b->cam;
   BCtrl init;
   std::memset(&init, 0, sizeof(init));

@@ -602,7 +602,8 @@ int swr_scene_set_transforms(swr_scene* s, const swr_object_transform* xf, uint3
   }
   std::copy(xf, xf + n, I->xf.begin());
   SWR_CUDA(cudaStreamSynchronize(stream));  // the host arrays above go out of scope
-  s->dev.ray_flags = swr::first_ray_flags(area[0] > 0.0 ? area[1] / area[0] : 0.0);
+  s->flat_share = area[0] > 0.0 ? area[1] / area[0] : 0.0;
+  s->dev.ray_flags = swr::first_ray_flags(s->flat_share);
   return SWR_OK;
 }
 

@@ -381,6 +381,7 @@ int swr_scene_create(const swr_scene_desc* d, const swr_build_opts* opts, swr_sc
     ds.num_slots = (uint32_t)pk.slot_to_id.size();
     ds.num_objects = d->num_objects;
     ds.num_tris = d->num_triangles;
+    s->flat_share = pk.flat_share;
     ds.ray_flags = swr::first_ray_flags(pk.flat_share);
     s->depth = pk.depth;
     s->node_bytes = (uint64_t)pk.num_nodes * 80;

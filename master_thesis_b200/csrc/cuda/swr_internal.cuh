@@ -49,6 +49,7 @@ struct swr_scene {
   size_t scratch_bytes = 0;
   uint32_t depth = 0;
   uint64_t node_bytes = 0, tri_bytes = 0;
+  double flat_share = 0.0;  // of the triangles' area, in triangles whose reference box is flat
   int device = 0;
   int num_sms = 0;
   std::vector<uint32_t> slot_to_id;  // host copy
@@ -69,7 +70,8 @@ int cuda_fail(cudaError_t err, const char* what);
     if (_e != cudaSuccess) return swr::cuda_fail(_e, #call); \
   } while (0)
 
-// DevScene::ray_flags by the share of the triangles' area whose reference boxes are flat
+// DevScene::ray_flags by the share of the triangles' area whose reference boxes are flat (a batch: its
+// scenes' shares weighted by their samples)
 uint32_t first_ray_flags(double flat_share);
 
 // true when p is host memory that the device cannot address directly

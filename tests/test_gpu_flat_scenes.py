@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import master_thesis_b200 as swr
+from master_thesis_b200 import _native as N
 from master_thesis_b200 import rt, scenes
 from master_thesis_b200.api import MAT_DTYPE
 from oracle import oracle as O
@@ -126,3 +127,28 @@ def test_moved_there_and_back(tmp_path):
     sc.set_transforms(home)
     back, back_visits = _visits(sc, o, d)
     assert torch.equal(back, hits) and back_visits == visits
+
+
+@pytest.mark.parametrize("flat_jobs", [0, 1, 3])
+def test_batches_of_flat_and_other_scenes(flat_jobs):
+    """The rays of all jobs of a batch start alike, by the jobs' share of flat walls; images and gradients are
+    those of each scene alone."""
+    import torch
+    W, H, spp, depth = 80, 60, 4, 4
+    jobs, adjoint = [], []
+    for k in range(4):
+        at = 8192.0 if k < flat_jobs else 0.0
+        sc = swr.Scene(_scene(at, False))
+        jobs.append(dict(scene=sc, cam=swr.make_camera((at + 3.0, 0.5, 0.25), (1.0, 0.0), W, H, fov_deg=60.0), width=W,
+                         height=H, spp=spp, depth=depth, seed=5 + k, mode=N.MODE_PHYSICAL))
+        adjoint.append(dict(jobs[-1], dl_dimage=torch.ones((H, W, 3), device="cuda")))
+    for kw in (dict(), dict(wave_size=4096)):
+        for j, img in zip(jobs, swr.Batch().render(jobs, **kw)):
+            want = j["scene"].render(j["cam"], W, H, spp, depth, seed=j["seed"], mode=N.MODE_PHYSICAL)
+            assert want.abs().sum() > 0
+            assert torch.allclose(img, want, rtol=1e-5, atol=1e-7)
+    for j, got in zip(jobs, swr.Batch().render_adjoint(adjoint)):
+        want = j["scene"].render_adjoint(j["cam"], W, H, spp, depth, torch.ones((H, W, 3), device="cuda"),
+                                         seed=j["seed"])
+        for g, w in zip(got, want):
+            assert torch.linalg.norm(g - w) <= 1e-4 * torch.linalg.norm(w)
