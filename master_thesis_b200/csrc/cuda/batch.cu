@@ -342,14 +342,15 @@ __device__ __forceinline__ unsigned begin_trace(const BArgs& A, BCtrl* __restric
 }
 
 // bounce traversal of a small shared queue, eight lanes per ray (swr_wide.cuh)
+template <bool kStrict>
 __global__ void __launch_bounds__(kTB) k_btrace_wide(BArgs A, BCtrl* __restrict__ ctrl, BQueue q, int parity) {
   __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
   const unsigned n = begin_trace(A, ctrl, parity);
   for (unsigned i = swrx::wide_first(); i < n; i += swrx::wide_stride()) {
     const float4 o = q.o[i], d = q.d[i];
     const DevScene& sc = A.scenes[A.jobs[__float_as_uint(q.c[i].w) >> 16].scene];
-    const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
-        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr, A.ray_flags);
+    const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference, kStrict>(
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, nullptr);
     if ((lane() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
   }
 }
@@ -786,7 +787,9 @@ int swr_render_batch(swr_batch* b, const swr_batch_job* jobs, uint32_t n, const 
   k_bcamera<<<bcamera_grid(num_sms, pixels), kTB, 0, stream>>>(A, dctrl);
   SWR_CUDA(cudaGetLastError());
   int per_sm = 0;
-  auto trace_kernel = capw <= swrx::kWideRays ? k_btrace_wide : k_btrace;  // the queue bounds every round
+  auto trace_kernel = k_btrace;
+  if (capw <= swrx::kWideRays)  // the queue bounds every round
+    trace_kernel = A.ray_flags ? k_btrace_wide<true> : k_btrace_wide<false>;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel, kTB, 0));
   const unsigned tgrid = (unsigned)(num_sms * std::max(per_sm, 1));
   int shade_per_sm = 0;

@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera(DevScene sc, Frame F, Ct
 }
 
 // The camera prefix of a chunk of few pixels, eight lanes per pixel (swr_wide.cuh).
+template <bool kStrict>
 __global__ void __launch_bounds__(kTraceBlock) k_camera_wide(DevScene sc, Frame F, Ctrl* __restrict__ ctrl) {
   __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
   const unsigned first = (lane_id() & 7u) == 0u;  // the lane that writes for its group
@@ -238,8 +239,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera_wide(DevScene sc, Frame 
     f3 o = mk(F.org[0], F.org[1], F.org[2]);
     float4 rec0 = make_float4(0, 0, 0, 0), rec1 = make_float4(0, 0, 0, __uint_as_float(kDeadSlot));
     for (uint32_t i = 0; i < F.depth; ++i) {
-      const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference>(
-          sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, o, d, stack, nullptr, sc.ray_flags);
+      const swrx::WideHit h = swrx::wide_closest<false, swrx::kRuleReference, kStrict>(
+          sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, o, d, stack, nullptr);
       traced += first;
       if (h.slot == kDeadSlot) break;
       const f3 p = swrx::hit_point(o, d, h.t);
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_camera_wide(DevScene sc, Frame 
 // Launches the camera kernel for the F.npix pixels of a chunk.
 static int launch_camera(const swr_scene* s, const Frame& F, Ctrl* ctrl, cudaStream_t st) {
   const bool wide = F.npix <= swrx::kWideRays;
-  auto kern = wide ? k_camera_wide : k_camera;
+  auto kern = !wide ? k_camera : s->dev.ray_flags ? k_camera_wide<true> : k_camera_wide<false>;
   int per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));
   const unsigned per_block = wide ? swrx::kWideGroups : kTraceBlock;
@@ -460,7 +461,7 @@ __device__ __forceinline__ void add_stats(Ctrl* __restrict__ ctrl, const swrx::T
 }
 
 // Bounce traversal of a small queue, eight lanes per ray (swr_wide.cuh).
-template <bool kStats>
+template <bool kStats, bool kStrict>
 __global__ void __launch_bounds__(kTraceBlock)
     k_trace_wide(DevScene sc, Frame F, Ctrl* __restrict__ ctrl, Queue q, int parity) {
   __shared__ uint2 stack[swrx::kWideGroups * swrx::kStackTotal];
@@ -468,9 +469,8 @@ __global__ void __launch_bounds__(kTraceBlock)
   swrx::TraceStats st{0, 0};
   for (unsigned i = swrx::wide_first(); i < n; i += swrx::wide_stride()) {
     const float4 o = q.o[i], d = q.d[i];
-    const swrx::WideHit h = swrx::wide_closest<kStats, swrx::kRuleReference>(
-        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, &st,
-        sc.ray_flags);
+    const swrx::WideHit h = swrx::wide_closest<kStats, swrx::kRuleReference, kStrict>(
+        sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), stack, &st);
     if ((lane_id() & 7u) == 0u) q.hit[i] = make_uint2(h.slot, __float_as_uint(h.t));
   }
   if (kStats) add_stats(ctrl, st);
@@ -1399,7 +1399,8 @@ int render_impl(swr_scene* s, const swr_camera* cam, const swr_render_opts* o, f
     default: return set_error(SWR_ERR_INVALID, "swr: trace_blocks must be 0, 9 or 10");
   }
   if (cap <= swrx::kWideRays && !postpone && o->trace_blocks == 0)  // bounds every round
-    trace_kernel = count ? k_trace_wide<true> : k_trace_wide<false>;
+    trace_kernel = s->dev.ray_flags ? (count ? k_trace_wide<true, true> : k_trace_wide<false, true>)
+                                    : (count ? k_trace_wide<true, false> : k_trace_wide<false, false>);
   if (static_fetch) trace_kernel = count ? k_trace<true> : k_trace<false>;
   if (o->refill > 32) return set_error(SWR_ERR_INVALID, "swr: refill must be 0..32");
   F.refill = o->refill ? o->refill : 8;

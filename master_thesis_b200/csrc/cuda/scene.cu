@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kTraceBlock, 10)
 }
 
 // The same for few rays, eight lanes each (swr_wide.cuh).
-template <bool kStats, int kRule>
+template <bool kStats, int kRule, bool kStrict>
 __global__ void __launch_bounds__(kTraceBlock)
     k_trace_closest_wide(DevScene sc, const float4* __restrict__ ro, const float4* __restrict__ rd, uint64_t n,
                          uint4* __restrict__ out, uint2* __restrict__ counts, unsigned long long*) {
@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(kTraceBlock)
     const float4 o = ro[i], d = rd[i];
     swrx::TraceStats st{0, 0};
     const swrx::WideHit h =
-        swrx::wide_closest<kStats, kRule>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, swrx::mk(o.x, o.y, o.z),
-                                          swrx::mk(d.x, d.y, d.z), stack, &st, sc.ray_flags);
+        swrx::wide_closest<kStats, kRule, kStrict>(sc.nodes, sc.tris, sc.tri_boxes, sc.obj_boxes, swrx::mk(o.x, o.y, o.z),
+                                                   swrx::mk(d.x, d.y, d.z), stack, &st);
     if (kStats) st.tris = __reduce_add_sync(0xFFu << (threadIdx.x & 24u), st.tris);
     if ((threadIdx.x & 7u) == 0u) {
       uint4 r = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, __float_as_uint(h.d2), __float_as_uint(h.t));
@@ -297,9 +297,14 @@ int trace_impl(swr_scene* s, const float* ray_o, const float* ray_d, uint64_t n,
   else if (counts)
     kern = few ? k_trace_closest<true, swrx::kRuleReference, true> : k_trace_closest<true, swrx::kRuleReference, false>;
   if (wide) {
-    kern = k_trace_closest_wide<false, swrx::kRuleReference>;
-    if (rule == swrx::kRuleRayQuery) kern = k_trace_closest_wide<false, swrx::kRuleRayQuery>;
-    else if (counts) kern = k_trace_closest_wide<true, swrx::kRuleReference>;
+    const bool strict = s->dev.ray_flags != 0u;
+    kern = strict ? k_trace_closest_wide<false, swrx::kRuleReference, true>
+                  : k_trace_closest_wide<false, swrx::kRuleReference, false>;
+    if (rule == swrx::kRuleRayQuery)
+      kern = k_trace_closest_wide<false, swrx::kRuleRayQuery, false>;
+    else if (counts)
+      kern = strict ? k_trace_closest_wide<true, swrx::kRuleReference, true>
+                    : k_trace_closest_wide<true, swrx::kRuleReference, false>;
   }
   int per_sm = 0;
   SWR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceBlock, 0));

@@ -33,11 +33,14 @@ struct WideHit {
 };
 
 // The calling lane's group works on one ray (o, d), the same in its eight lanes; mem: the block's
-// rows, of which the group uses its own kStackTotal entries; flags: as Traversal::init.
-template <bool kStats, int kRule>
+// rows, of which the group uses its own kStackTotal entries. kStrict: the slab tests are made on every
+// candidate from the start (DevScene::ray_flags; a template parameter, since a flag read at run time took
+// one more register, which these kernels spill: 12,000 queries of the tessellated Cornell box 37.8 against
+// 37.0 us).
+template <bool kStats, int kRule, bool kStrict>
 __device__ __forceinline__ WideHit wide_closest(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                                              const float* __restrict__ tri_boxes, const float* __restrict__ obj_boxes,
-                                             f3 o, f3 d, uint2* mem, TraceStats* stats, uint32_t flags) {
+                                             f3 o, f3 d, uint2* mem, TraceStats* stats) {
   const uint32_t c = threadIdx.x & 7u, shift = threadIdx.x & 24u;
   const uint32_t gmask = 0xFFu << shift;
   uint2* stack = mem + (threadIdx.x / kWideLanes) * kStackTotal;
@@ -50,7 +53,7 @@ __device__ __forceinline__ WideHit wide_closest(const float4* __restrict__ nodes
   const uint32_t nx = 32u + c + ((oct & 1u) ? 24u : 0u), fx = 32u + c + ((oct & 1u) ? 0u : 24u);
   const uint32_t ny = 40u + c + ((oct & 2u) ? 24u : 0u), fy = 40u + c + ((oct & 2u) ? 0u : 24u);
   const uint32_t nz = 48u + c + ((oct & 4u) ? 24u : 0u), fz = 48u + c + ((oct & 4u) ? 0u : 24u);
-  for (bool strict = kRule == kRuleReference && (flags & Traversal::kStrict);; strict = true) {
+  for (bool strict = kStrict;; strict = true) {
     uint32_t bslot = 0xFFFFFFFFu, bkey = 0xFFFFFFFFu;
     float bt = INFINITY, bd2 = INFINITY, tprune = INFINITY;
     uint2 ng = make_uint2(0u, (1u << (24 + oct)) | 1u);

@@ -152,3 +152,16 @@ def test_batches_of_flat_and_other_scenes(flat_jobs):
                                          seed=j["seed"])
         for g, w in zip(got, want):
             assert torch.linalg.norm(g - w) <= 1e-4 * torch.linalg.norm(w)
+
+
+@pytest.mark.parametrize("at", [0.0, 8192.0])
+def test_counted_queries(at):
+    """Queries that count their nodes and triangles, few (eight lanes each) and many, find the same hits."""
+    import torch
+    sc = swr.Scene(_scene(at, False))
+    o, d = scenes.uniform_rays(30000, (at - 2, -4, -4), (at + 6, 4, 4), 5)
+    want = sc.trace(o, d)
+    for n in (30000, 5000):
+        counts = torch.zeros((n, 2), dtype=torch.int32, device="cuda")
+        assert torch.equal(sc.trace(o[:n], d[:n], counts=counts), want[:n])
+        assert int(counts[:, 0].min()) >= 1
